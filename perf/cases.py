@@ -164,3 +164,68 @@ def tolerance(case):
     if case["dtype"] == "bf16":
         return {"rel": 3.8e-3, "max": 3.2e-2}
     return {"rel": 1.4e-3, "max": 7e-3}
+
+
+def _quantised(x, group, factor):
+    """int8 values (as float64) and one scale per `group` rows of x [..., rows, head_dim], which is first multiplied by `factor`."""
+    rows = x.shape[-2]
+    x = torch.nn.functional.pad(x.float(), (0, 0, 0, -rows % group)).unflatten(-2, (-1, group))
+    largest = (x * factor).abs().amax((-1, -2), keepdim=True).clamp_min(1e-7)
+    y = x * (127.0 / largest * factor)
+    values = torch.trunc(y + torch.where(y < 0, -0.5, 0.5)).clamp(-128, 127)
+    scale = (largest / 127.0).expand(*x.shape[:-1], 1)
+    return values.double().flatten(-3, -2)[..., :rows, :], scale.double().flatten(-3, -2)[..., :rows, :]
+
+
+def _un_quantised(case):
+    """The documented choice between the un-quantised and the INT8 kernel, by the length of K."""
+    if case["call"] == "sageattn_quantized_kv":
+        return False
+    q_len, kv_len = case["q_len"], case["kv_len"]
+    if case["head_dim"] == 64:
+        if case["causal"] or q_len < kv_len:
+            return kv_len <= 6144
+        return kv_len <= (2048 if case["layout"] == "HND" else 3072)
+    return kv_len <= (4096 if q_len * 2 < kv_len else 2048)
+
+
+def exact(case, seed):
+    """The softmax and both products in 64 bits, on the values that the path is defined on: the int8 values and scales of
+    Q and K (the inputs in 16 bits for the un-quantised kernel) and V in fp16."""
+    made = dict(case, call="sageattn")
+    state = prepare(made, seed)
+    q, k, v = (state[n].half() if case["dtype"] == "fp32" else state[n] for n in "qkv")
+    if case["layout"] == "NHD":
+        q, k, v = (t.transpose(1, 2) for t in (q, k, v))
+    dim, rep = case["head_dim"], case["heads"] // case["kv_heads"]
+    sm_scale, log2e = dim ** -0.5, torch.tensor(math.log2(math.e), dtype=torch.float32)
+    factor = (torch.tensor(sm_scale, dtype=torch.float32) * log2e).item()
+    out = torch.empty(q.shape, dtype=torch.float64, device=q.device)
+    lse = torch.empty(q.shape[:3], dtype=torch.float64, device=q.device)
+    for b in range(case["batch"]):
+        for h in range(case["heads"]):
+            qh, kh, vh = q[b, h], k[b, h // rep], v[b, h // rep].half().double()
+            shift = None
+            if _un_quantised(case):
+                qh, kh = qh.double() * factor, kh.double()
+            else:
+                if case["smooth_k"]:
+                    mean = kh.float().mean(0).to(kh.dtype)
+                    shift = qh.double() @ mean.double() * sm_scale
+                    kh = kh.float() - mean.float()
+                (qi, qs), (ki, ks) = _quantised(qh, 32, factor), _quantised(kh, 16, 1.0)
+                qh, kh = qi * qs, ki * ks
+            for r in range(0, case["q_len"], 4096):
+                s = qh[r:r + 4096] @ kh.T
+                if case["causal"]:
+                    s.masked_fill_(torch.ones(s.shape, dtype=torch.bool, device=s.device).triu_(r + 1), -math.inf)
+                top = s.amax(1, keepdim=True)
+                s = s.sub_(top).mul_(math.log(2.0)).exp_()
+                total = s.sum(1, keepdim=True)
+                out[b, h, r:r + 4096] = s @ vh / total
+                lse[b, h, r:r + 4096] = (top[:, 0] * math.log(2.0)) + total[:, 0].log()
+            if shift is not None:
+                lse[b, h] += shift
+    if case["layout"] == "NHD":
+        out = out.transpose(1, 2).contiguous()
+    return (out, lse) if case["lse"] else out
