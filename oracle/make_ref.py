@@ -36,7 +36,7 @@ FILES = {
 def make_ref(reference_dir: Path = DEFAULT_REFERENCE) -> bool:
     """Returns True when ``oracle/_ref/`` holds the files afterwards."""
     reference_dir = Path(reference_dir)
-    if not reference_dir.is_dir():
+    if not all((reference_dir / src).is_file() for src in FILES):
         return have_ref()
     REF_OUT.mkdir(exist_ok=True)
     for src, dst in FILES.items():
