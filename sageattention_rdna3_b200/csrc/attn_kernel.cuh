@@ -317,7 +317,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       tma_load_3d(s_k + stage * L::kKBytes, &tm_k, k_full + stage, 0, tile * kBlockN, g.b * p.Hkv + g.hkv);
     }
   };
-  if (warp == 4 && lane == 0) {
+  if (warp == 4 && elect_one()) {
     // The producer thread sets the barriers up itself and starts the first loads (Q and K tile 0,
     // which wait for nothing) at once, so their latency overlaps the TMEM allocation and the
     // CTA-wide barrier below.
@@ -363,15 +363,9 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const bool dead_on_arrival = *abort_flag != 0;
 
 // A failed wait records which barrier it was and leaves the role's loop.
-#ifndef SAGE_HINT_TMA
-#define SAGE_HINT_TMA true
-#endif
-#ifndef SAGE_HINT_MMA
-#define SAGE_HINT_MMA true
-#endif
-#ifndef SAGE_HINT_SOFTMAX
-#define SAGE_HINT_SOFTMAX true
-#endif
+// The producer's waits carry a suspend-time hint (it waits for most of the time); the waits of the MMA
+// and softmax warps, which are on the chain from scores to P and back, do not: plain try_wait wakes up
+// sooner (878 against 892 us for 37 heads of 8192 x 8192, head_dim 128).
 #define SAGE_WAIT_ROLE_OR(hinted, bar_ptr, parity, bar_id, action)   \
   if (!mbar_wait<hinted>((bar_ptr), (parity), abort_flag, p.wait_limit_cycles)) { \
     atomicCAS(fail_code, 0, kStatusWaitTimeout + 16 * (bar_id));    \
@@ -383,10 +377,10 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // nothing to do: the first loads of the producer land during the teardown wait
   } else if (warp == 4) {
     // ------------------------------------------------------------------ TMA producer
-    constexpr bool kHintRole = SAGE_HINT_TMA;
+    constexpr bool kHintRole = true;
     // Per segment: Q, K(first tile), then for every tile K(j+1) before V(j): K is needed first.  Q and
     // K of the CTA's first segment are already on their way.
-    if (lane == 0) {
+    if (elect_one()) {
       SegIter<CAUSAL, STREAMK> iter(p);
       Segment g;
       int kt = 0, it = 0;                 // KV tiles / segments so far (constant 0 unless STREAMK)
@@ -444,10 +438,10 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     __syncwarp();
   } else if (warp == 5) {
     // ------------------------------------------------------------------ MMA issuer
-    constexpr bool kHintRole = SAGE_HINT_MMA;
+    constexpr bool kHintRole = false;
     // Program order of the tensor pipe: QK(0,0) QK(0,1) | PV(0,0) QK(1,0) PV(0,1) QK(1,1) | ...
     // so the scores of the next half are ready while the softmax warps work on the current one.
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t kIdescQK = umma_idesc(2, 1, 1, 0, 0, kBlockM, kHalfN);   // s32 = s8 x s8
       constexpr uint32_t kIdescPV = umma_idesc(1, 0, 0, 0, 1, kBlockM, D);        // f32 = f16 x f16, V MN-major
       constexpr uint32_t kSwzQK = (D == 128) ? kSwizzle128B : kSwizzle64B;
@@ -549,7 +543,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ softmax / epilogue
-    constexpr bool kHintRole = SAGE_HINT_SOFTMAX;
+    constexpr bool kHintRole = false;
     bool yields = false;
     // (not in the persistent variant: its CTAs are given equal spans and must run at equal speed)
     if (SAGE_DEPHASE && !STREAMK) {

@@ -21,6 +21,20 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// True in one thread of the (converged) warp.  tcgen05.mma, tcgen05.commit and the TMA instructions take
+// their operands from uniform registers: inside a branch on elect.sync the compiler knows that one
+// thread is active and moves them over directly; behind `lane == 0` it emits a loop over the active
+// lanes around every such instruction (measured: about 100 clocks per tcgen05.mma against 25).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier ---------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
