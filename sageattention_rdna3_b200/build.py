@@ -65,7 +65,7 @@ def _run(cmd) -> None:
 
 def build_abi(force: bool = False, verbose: bool = False) -> Path:
     sources = [CSRC / "sage_abi.cu", CSRC / "attn_kernel.cuh", CSRC / "prep_kernels.cuh", CSRC / "merge_kernels.cuh",
-               CSRC / "ptx_sm100.cuh",
+               CSRC / "ptx_sm100.cuh", CSRC / "internal.h",
                REPO_DIR / "include" / "sage_b200.h"]
     if force or not _up_to_date(LIB_ABI, sources):
         cmd = [_nvcc(), *NVCC_FLAGS, "-o", str(LIB_ABI), str(CSRC / "sage_abi.cu")]
@@ -80,7 +80,7 @@ def build_ops(force: bool = False) -> Path:
     import torch
     from torch.utils import cpp_extension
 
-    sources = [CSRC / "torch_ops.cpp", REPO_DIR / "include" / "sage_b200.h"]
+    sources = [CSRC / "torch_ops.cpp", CSRC / "internal.h", REPO_DIR / "include" / "sage_b200.h"]
     extra = torch.__version__
     if force or not _up_to_date(LIB_OPS, sources, extra):
         torch_lib = Path(torch.__file__).parent / "lib"

@@ -252,10 +252,7 @@ def sageattn(
         o = out[0]
         if want_lse and smooth:
             # the kernel saw k - mean: every score of a row was lowered by sm_scale * q.mean
-            rep = q_shape[head_dim_idx] // k_shape[head_dim_idx]
-            km = out[1].float().repeat_interleave(rep, dim=1)                   # [B,Hq,D]
-            eq = "bhsd,bhd->bhs" if tensor_layout == "HND" else "bshd,bhd->bhs"
-            lse += torch.einsum(eq, q.float(), km) * sm_scale
+            ops.lse_add_q_mean(lse, q, out[1], layout, sm_scale)
         if os.environ.get("SAGEATTN_B200_CHECK_STATUS", "0") == "1":
             check_status(q.device)
 

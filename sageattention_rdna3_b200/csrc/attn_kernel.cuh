@@ -69,7 +69,9 @@ struct AttnParams {
   void* o;                      // caller layout; fp16 or bf16
   long long o_stride_b, o_stride_h, o_stride_s;   // elements
   int B, Hq, Hkv, Sq, Skv;
-  int q_groups, k_groups;
+  int q_groups, k_groups;       // 32-row groups of q_scale per head of the caller, 16-row groups of k_scale
+  int q_fold;                   // query heads of the caller in one "head" of this launch (1 unless folded):
+  int q_rows;                   // ... row r of it is row r % q_rows of head r / q_rows
   int n_q_tiles;
   int head_group;               // (batch, head) pairs scheduled together (a multiple of Hq/Hkv)
   int out_bf16;
@@ -566,11 +568,13 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     while (ok && iter.next(sg)) {
     const int bh = sg.bh, b = sg.b, hq = sg.hq, hkv = sg.hkv, q_base = sg.q_base, n_kv = sg.n_kv;
     const int row = q_base + threadIdx.x;
-    const int q_grp = (q_base + warp * 32) / 32;
     float qs = 0.0f;
     const float* ks_base = nullptr;
     if constexpr (!QKF) {
-      qs = (q_grp < p.q_groups) ? __ldg(p.q_scale + static_cast<long long>(bh) * p.q_groups + q_grp) : 0.0f;
+      if (row < p.Sq) {
+        const int head = row / p.q_rows;                // 0 unless folded
+        qs = __ldg(p.q_scale + (static_cast<long long>(bh) * p.q_fold + head) * p.q_groups + (row - head * p.q_rows) / 32);
+      }
       ks_base = p.k_scale + static_cast<long long>(b * p.Hkv + hkv) * p.k_groups;
     }
 

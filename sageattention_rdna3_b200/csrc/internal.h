@@ -1,0 +1,28 @@
+// Shared by libsage_b200.so (sage_abi.cu) and _C.so (torch_ops.cpp); not part of the public C ABI.
+#pragma once
+
+#include <stdint.h>
+
+#include "../../include/sage_b200.h"
+
+// Rows of a tile that are padding: a 128-row tile holds rows of one head, and with few queries per head
+// (some new tokens against a cached prefix) much of it is empty.  The query heads of a GQA group share
+// K and V, so without a causal mask their rows can share tiles too: the group becomes one head of
+// Hq/Hkv * Sq rows.  The int8 Q and the log-sum-exp are contiguous in that order; the output has to be
+// as well (its row stride runs on into the next head).  Returns how many heads become one, 1 for none;
+// folded wherever that gives fewer tiles (same work per tile, fewer of them: 32 heads of 64 rows on 8
+// kv heads are 16 tiles instead of 32).
+static inline int sage_gqa_fold(int64_t Hq, int64_t Hkv, int64_t Sq, int64_t o_stride_h, int64_t o_stride_s, int64_t is_causal) {
+  if (is_causal || Hkv <= 0 || Hq <= Hkv || Hq % Hkv != 0 || Sq <= 0) return 1;
+  const int64_t rep = Hq / Hkv, rows = rep * Sq;
+  if (rows > 0x3fffffff || o_stride_h != Sq * o_stride_s) return 1;
+  return (rows + 127) / 128 < rep * ((Sq + 127) / 128) ? (int)rep : 1;
+}
+
+extern "C" {
+// lse[b,h,s] += sm_scale * q[b,h,s,:] . k_mean[b, h / (Hq/Hkv), :], in fp32: refers the log-sum-exp of a
+// launch on centred keys (smooth_k) to the original ones.  lse: contiguous [B,Hq,Sq]; k_mean:
+// contiguous [B,Hkv,D] in the dtype of q.
+int sage_lse_add_q_mean(const sage_strided_t* q, int dtype, const void* k_mean, float* lse, int B, int Hq, int Hkv, int Sq,
+                        int D, float sm_scale, void* stream);
+}

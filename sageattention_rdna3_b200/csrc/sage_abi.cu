@@ -14,6 +14,7 @@
 #include <mutex>
 
 #include "attn_kernel.cuh"
+#include "internal.h"
 #include "merge_kernels.cuh"
 #include "prep_kernels.cuh"
 
@@ -145,6 +146,7 @@ void fill_attn_params(sage::AttnParams* pp, void* o, int64_t o_stride_b, int64_t
   p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.Sq = Sq; p.Skv = Skv;
   p.q_groups = (Sq + sage::kQGroupRows - 1) / sage::kQGroupRows;
   p.k_groups = (Skv + sage::kKGroupRows - 1) / sage::kKGroupRows;
+  p.q_fold = 1; p.q_rows = Sq;
   p.n_q_tiles = (Sq + sage::kBlockM - 1) / sage::kBlockM;
   // 8 heads at a time (each needs Skv * D * 3 bytes of K and V in L2), whole GQA groups only
   const int rep = Hq / Hkv;
@@ -669,9 +671,18 @@ int attn_int8_impl(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (Sq == 0) return SAGE_OK;
 
+  const int fold = (s_dump == nullptr && n_peers == 0) ? sage_gqa_fold(Hq, Hkv, Sq, o_stride_h, o_stride_s, is_causal) : 1;
+  const int rows_per_head = Sq;
+  if (fold > 1) {
+    Hq /= fold;
+    Sq *= fold;
+    o_stride_h *= fold;
+  }
   sage::AttnParams p;
   fill_attn_params(&p, o, o_stride_b, o_stride_h, o_stride_s, out_dtype, B, Hq, Hkv, Sq, Skv, lse, status);
   p.q_scale = q_scale; p.k_scale = k_scale;
+  p.q_fold = fold; p.q_rows = rows_per_head;
+  p.q_groups = (rows_per_head + sage::kQGroupRows - 1) / sage::kQGroupRows;
   p.s_dump = s_dump;
   p.n_peers = n_peers;                                  // (the persistent launch does not scatter: plain launch)
   for (int i = 0; i < n_peers; ++i) p.peer_o[i] = peer_o[i];
@@ -753,6 +764,33 @@ int attn_int8_impl(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t*
 #undef SAGE_LAUNCH
 }
 }  // namespace
+
+int sage_lse_add_q_mean(const sage_strided_t* q, int dtype, const void* k_mean, float* lse, int B, int Hq, int Hkv, int Sq,
+                        int D, float sm_scale, void* stream) {
+  SAGE_REQUIRE(q && q->ptr && k_mean && lse, "sage_lse_add_q_mean: null pointer");
+  SAGE_REQUIRE(dtype == SAGE_DTYPE_F16 || dtype == SAGE_DTYPE_BF16, "sage_lse_add_q_mean: q must be f16 or bf16");
+  SAGE_REQUIRE(D == 64 || D == 128, "sage_lse_add_q_mean: head_dim must be 64 or 128, got %d", D);
+  SAGE_REQUIRE(B >= 0 && Hq >= 0 && Hkv > 0 && Hq % Hkv == 0 && Sq >= 0, "sage_lse_add_q_mean: bad sizes");
+  SAGE_REQUIRE(aligned16(q->ptr) && strides_ok(q) && aligned16(k_mean),
+               "sage_lse_add_q_mean: q and the mean need 16-byte aligned bases and strides % 8 == 0");
+  const long long rows = static_cast<long long>(B) * Hq * Sq;
+  if (rows == 0) return SAGE_OK;
+  const long long blocks = (rows * (D / 8) + 255) / 256;
+  if (blocks > 0x7fffffffLL) return fail(SAGE_ERR_INVALID, "too many rows for one launch (%lld)", rows);
+  const sage::StridedView v = view_of(q);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define SAGE_LSE_MEAN(T, DD)                                                                                   \
+  sage::sage_lse_mean_kernel<T, DD><<<static_cast<unsigned>(blocks), 256, 0, st>>>(v, static_cast<const T*>(k_mean), lse, Hq, \
+                                                                                   Hq / Hkv, Sq, rows, sm_scale)
+  if (dtype == SAGE_DTYPE_BF16) {
+    if (D == 128) SAGE_LSE_MEAN(__nv_bfloat16, 128); else SAGE_LSE_MEAN(__nv_bfloat16, 64);
+  } else {
+    if (D == 128) SAGE_LSE_MEAN(__half, 128); else SAGE_LSE_MEAN(__half, 64);
+  }
+#undef SAGE_LSE_MEAN
+  SAGE_CUDA(cudaGetLastError());
+  return SAGE_OK;
+}
 
 int sage_fold_attn_partial(const sage_strided_t* o_acc, float* lse_acc, int64_t lse_stride_b, int64_t lse_stride_h,
                            const sage_strided_t* o_part, int part_dtype, const float* lse_part, int B, int H, int S, int D,

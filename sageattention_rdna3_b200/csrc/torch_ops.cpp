@@ -13,7 +13,7 @@
 
 #include <vector>
 
-#include "../../include/sage_b200.h"
+#include "internal.h"
 
 namespace {
 
@@ -263,7 +263,9 @@ at::Tensor qk_int8_sv_f16_attn(const at::Tensor& q_i8, const at::Tensor& k_i8, c
   }
   // Problems that would fill the GPU unevenly run on persistent CTAs and need scratch for partial results.
   at::Tensor workspace;
-  const int64_t ws_bytes = dump_ptr ? 0 : sage_attn_workspace_bytes((int)B, (int)Hq, (int)Sq, (int)Skv, (int)D, (int)is_causal);
+  const int64_t fold = sage_gqa_fold(Hq, Hkv, Sq, os.stride_h, os.stride_s, is_causal);   // as the launcher does
+  const int64_t ws_bytes =
+      dump_ptr ? 0 : sage_attn_workspace_bytes((int)B, (int)(Hq / fold), (int)(Sq * fold), (int)Skv, (int)D, (int)is_causal);
   if (ws_bytes > 0) workspace = at::empty({ws_bytes}, q_i8.options().dtype(at::kByte));
   check_rc(sage_qk_int8_sv_f16_attn_ws(q_i8.data_ptr<int8_t>(), k_i8.data_ptr<int8_t>(), &vs, o.data_ptr(), os.stride_b,
                                        os.stride_h, os.stride_s, q_scale.data_ptr<float>(),
@@ -393,6 +395,24 @@ std::vector<at::Tensor> sageattn_fwd(const at::Tensor& q, const at::Tensor& k, c
   return {o};
 }
 
+// lse_add_q_mean(Tensor(a!) lse, Tensor query, Tensor key_mean, int tensor_layout, float sm_scale) -> ()
+// lse [B,Hq,Sq] += sm_scale * q.mean(k): refers the log-sum-exp of centred keys to the original ones.
+void lse_add_q_mean(at::Tensor& lse, const at::Tensor& q, const at::Tensor& k_mean, int64_t layout, double sm_scale) {
+  check_16b(q, "query");
+  const Dims d = dims_of(q, layout);
+  TORCH_CHECK(lse.is_cuda() && lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.numel() == d.B * d.H * d.S,
+              "lse must be a contiguous fp32 CUDA tensor [B,Hq,Sq]");
+  TORCH_CHECK(k_mean.is_contiguous() && k_mean.dim() == 3 && k_mean.size(0) == d.B && k_mean.size(2) == d.D &&
+                  k_mean.size(1) > 0 && d.H % k_mean.size(1) == 0 && k_mean.scalar_type() == q.scalar_type() &&
+                  k_mean.device() == q.device(),
+              "key_mean must be a contiguous [B,Hkv,D] tensor of the input dtype");
+  c10::cuda::CUDAGuard guard(q.device());
+  const sage_strided_t qs = strided_of(q, layout);
+  check_rc(sage_lse_add_q_mean(&qs, dtype_code(q), k_mean.data_ptr(), lse.data_ptr<float>(), (int)d.B, (int)d.H,
+                               (int)k_mean.size(1), (int)d.S, (int)d.D, static_cast<float>(sm_scale), current_stream(q)),
+           "lse_add_q_mean");
+}
+
 // fold_partial(Tensor(a!) o_acc, Tensor(b!) lse_acc, Tensor o_part, Tensor lse_part, int tensor_layout, int first) -> ()
 // One launch that folds a partial result (o_part fp16 / bf16 in `tensor_layout`, lse_part fp32 [B,H,S])
 // into fp32 accumulators (o_acc in `tensor_layout`, lse_acc [B,H,S]; both may be row slices of larger
@@ -435,6 +455,7 @@ TORCH_LIBRARY(sageattention, m) {
         "-> Tensor[]");
   m.def("prep_smooth_qkv(Tensor query, Tensor key, Tensor? value, int tensor_layout, float sm_scale) -> Tensor[]");
   m.def("mean_seq(Tensor input, int tensor_layout) -> Tensor");
+  m.def("lse_add_q_mean(Tensor(a!) lse, Tensor query, Tensor key_mean, int tensor_layout, float sm_scale) -> ()");
   m.def("v_to_f16(Tensor value, int tensor_layout) -> Tensor");
 }
 
@@ -448,6 +469,7 @@ TORCH_LIBRARY_IMPL(sageattention, CUDA, m) {
   m.impl("fold_partial", &fold_partial);
   m.impl("prep_smooth_qkv", &prep_smooth_qkv);
   m.impl("mean_seq", &mean_seq);
+  m.impl("lse_add_q_mean", &lse_add_q_mean);
   m.impl("v_to_f16", &v_to_f16);
 }
 

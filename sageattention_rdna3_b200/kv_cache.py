@@ -118,7 +118,5 @@ def sageattn_quantized_kv(q: torch.Tensor, kv: QuantizedKV, is_causal: bool = Fa
         ops.qk_int8_sv_f16_attn(q_int8, kv.k_int8, kv.v16, o, q_scale, kv.k_scale, layout, int(is_causal), sm_scale,
                                 value_layout=kv.v_layout, status=_status_word(q.device), lse=lse)
         if return_lse and kv.k_mean is not None:
-            km = kv.k_mean.float().repeat_interleave(Hq // kv.num_kv_heads, dim=1)
-            eq = "bhsd,bhd->bhs" if tensor_layout == "HND" else "bshd,bhd->bhs"
-            lse += torch.einsum(eq, q.float(), km) * sm_scale
+            ops.lse_add_q_mean(lse, q, kv.k_mean, layout, sm_scale)
     return (o, lse) if return_lse else o
