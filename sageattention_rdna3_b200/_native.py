@@ -125,6 +125,13 @@ def load_ops():
     return _ops
 
 
+def load_module():
+    """The extension as a Python module: the short way into ``sageattn_fwd`` (``csrc/torch_ops.cpp``)."""
+    load_ops()
+    from . import _C
+    return _C
+
+
 def native_available() -> bool:
     try:
         load_ops()

@@ -92,7 +92,7 @@ def build_ops(force: bool = False) -> Path:
             cmd += ["-isystem", str(inc)]
         cmd += [str(CSRC / "torch_ops.cpp"), "-o", str(LIB_OPS),
                 f"-L{PKG_DIR}", "-l:libsage_b200.so", f"-L{torch_lib}",
-                "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda",
+                "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda", "-ltorch_python",
                 "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
         _run(cmd)
         _write_stamp(LIB_OPS, sources, extra)

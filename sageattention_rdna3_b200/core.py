@@ -58,6 +58,23 @@ def _status_mirror(device: torch.device):
 _MIRROR_ON = os.environ.get("SAGEATTN_B200_STATUS_MIRROR", "1") != "0"
 
 
+# The short way into the operator for plain calls (csrc/torch_ops.cpp); set, and the device registered
+# with it, by the first call that took the long way.
+_plain_call = None
+_registered = set()
+
+
+def _register(device: torch.device) -> None:
+    global _plain_call
+    idx = device.index if device.index is not None else torch.cuda.current_device()
+    if idx in _registered:
+        return
+    module = _native.load_module()
+    module.register_device(idx, _status_word(device), _status_mirror(device)[0] if _MIRROR_ON else None)
+    _registered.add(idx)
+    _plain_call = module.sageattn_plain
+
+
 def check_status(device: Union[torch.device, int, str, None] = None) -> None:
     """Synchronise and raise if a kernel on ``device`` reported an internal error since the last check."""
     if device is None:
@@ -164,6 +181,10 @@ def sageattn(
     tensor, and ``scatter_to`` (device addresses of further copies of ``out``, normally in other
     GPUs' memory, see :mod:`.peer_gather`) makes the kernel write them as well.
     """
+    if _plain_call is not None and not kwargs and not return_lse and not torch.compiler.is_compiling():
+        o = _plain_call(q, k, v, tensor_layout, is_causal, sm_scale, smooth_k)
+        if o is not None:                # None: not a plain call, or one that the checks below refuse
+            return o
     dtype = q.dtype
     assert q.is_cuda, "Input tensors must be on CUDA/HIP device."
     assert dtype in [torch.float16, torch.bfloat16, torch.float32], (
@@ -224,7 +245,9 @@ def sageattn(
     want_lse = return_lse and os.environ.get("SAGEATTN_B200_LSE_ZEROS", "0") != "1"
     if return_lse:
         lse_shape = (q_shape[0], q_shape[head_dim_idx], q_len)
-        if want_lse:
+        if want_lse and kv_len > 0:      # the launch writes every row
+            lse = torch.empty(lse_shape, dtype=torch.float32, device=q.device)
+        elif want_lse:
             lse = torch.full(lse_shape, float("-inf"), dtype=torch.float32, device=q.device)
         else:
             lse = torch.zeros(lse_shape, dtype=torch.float32, device=q.device)
@@ -246,6 +269,7 @@ def sageattn(
                 seen[0] = 0
                 _status_word(q.device).zero_()
                 raise RuntimeError(_STATUS_MESSAGE.format(code=code) + "; reported by the call after the one that failed")
+        _register(q.device)
         out = ops.sageattn_fwd(q, k, v, layout, int(is_causal), sm_scale, int(smooth), int(direct),
                                _status_word(q.device), lse if want_lse else None, out_arg,
                                [int(a) for a in scatter_to] if scatter_to else None)

@@ -4,13 +4,20 @@
 // declared in csrc/attn_gfx11.h.  `tensor_layout`: 0 = NHD [B,S,H,D], 1 = HND [B,H,S,D]
 // (csrc/attn_gfx11.cu:32-33).
 #include <Python.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/TensorSubclassLikeUtils.h>
+#include <ATen/core/dispatch/Dispatcher.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 #include <torch/types.h>
 
 #include <cuda_runtime.h>
 
+#include <cmath>
+#include <cstdlib>
 #include <vector>
 
 #include "internal.h"
@@ -413,6 +420,41 @@ void lse_add_q_mean(at::Tensor& lse, const at::Tensor& q, const at::Tensor& k_me
            "lse_add_q_mean");
 }
 
+// sageattn_kv_fwd(Tensor query, Tensor key, Tensor k_scale, Tensor value, Tensor? key_mean, int tensor_layout,
+//                 int value_layout, int is_causal, float sm_scale, Tensor status, int want_lse) -> Tensor[]
+// sageattn against keys and values that were quantised before: quantise Q, attention, and with want_lse
+// the log-sum-exp (referred to the original keys when there is a mean).  Returns [output] or
+// [output, lse].  One Python -> C++ crossing instead of three, no fill of the log-sum-exp (the
+// launch writes every row).
+std::vector<at::Tensor> sageattn_kv_fwd(const at::Tensor& q, const at::Tensor& k_i8, const at::Tensor& k_scale,
+                                        const at::Tensor& v, const c10::optional<at::Tensor>& k_mean, int64_t layout,
+                                        int64_t value_layout, int64_t is_causal, double sm_scale, const at::Tensor& status,
+                                        int64_t want_lse) {
+  check_16b(q, "query");
+  const Dims dq = dims_of(q, layout);
+  TORCH_CHECK(k_i8.dim() == 4 && k_i8.size(0) == dq.B && k_i8.size(3) == dq.D && k_i8.size(1) > 0 && k_i8.size(2) > 0 &&
+                  dq.H % k_i8.size(1) == 0 && dq.B > 0 && dq.H > 0 && dq.S > 0,
+              "sageattn_kv_fwd: query and key shapes do not match, or one is empty");
+  c10::cuda::CUDAGuard guard(q.device());
+  at::Tensor o = at::empty_like(q);
+  at::Tensor q_i8 = at::empty({dq.B, dq.H, dq.S, dq.D}, q.options().dtype(at::kChar));
+  at::Tensor q_scale = at::empty({dq.B, dq.H, (dq.S + 31) / 32}, q.options().dtype(at::kFloat));
+  c10::optional<at::Tensor> lse;
+  if (want_lse) lse = at::empty({dq.B, dq.H, dq.S}, q.options().dtype(at::kFloat));
+  const sage_strided_t qs = strided_of(q, layout);
+  sage_strided_t none_k = qs;                            // no keys: only the Q blocks of the launch exist
+  check_rc(sage_quant_qk_int8(&qs, &none_k, nullptr, nullptr, nullptr, dtype_code(q), (int)dq.B, (int)dq.H,
+                              (int)k_i8.size(1), (int)dq.S, 0, (int)dq.D, static_cast<float>(sm_scale),
+                              q_i8.data_ptr<int8_t>(), q_scale.data_ptr<float>(), nullptr, nullptr, current_stream(q)),
+           "sageattn_kv_fwd");
+  const c10::optional<at::Tensor> st(status), none;
+  qk_int8_sv_f16_attn(q_i8, k_i8, v, o, q_scale, k_scale, layout, is_causal, sm_scale, value_layout, none, st, lse,
+                      c10::nullopt);
+  if (!want_lse) return {o};
+  if (k_mean.has_value()) lse_add_q_mean(*lse, q, *k_mean, layout, sm_scale);
+  return {o, *lse};
+}
+
 // fold_partial(Tensor(a!) o_acc, Tensor(b!) lse_acc, Tensor o_part, Tensor lse_part, int tensor_layout, int first) -> ()
 // One launch that folds a partial result (o_part fp16 / bf16 in `tensor_layout`, lse_part fp32 [B,H,S])
 // into fp32 accumulators (o_acc in `tensor_layout`, lse_acc [B,H,S]; both may be row slices of larger
@@ -443,6 +485,8 @@ TORCH_LIBRARY(sageattention, m) {
   m.def("fold_partial(Tensor(a!) o_acc, Tensor(b!) lse_acc, Tensor o_part, Tensor lse_part, int tensor_layout, int first) -> ()");
   m.def("sageattn_fwd(Tensor query, Tensor key, Tensor value, int tensor_layout, int is_causal, float sm_scale, "
         "int smooth_k, int use_direct, Tensor status, Tensor? lse=None, Tensor? out=None, int[]? peer_ptrs=None) -> Tensor[]");
+  m.def("sageattn_kv_fwd(Tensor query, Tensor key, Tensor k_scale, Tensor value, Tensor? key_mean, int tensor_layout, "
+        "int value_layout, int is_causal, float sm_scale, Tensor status, int want_lse) -> Tensor[]");
   m.def("fp16_attn(Tensor query, Tensor key, Tensor value, Tensor(a!) output, int tensor_layout, int value_layout, "
         "int is_causal, float sm_scale, int bm_sel=0, Tensor? status=None, Tensor? lse=None) -> Tensor");
   m.def("bf16_attn(Tensor query, Tensor key, Tensor value, Tensor(a!) output, int tensor_layout, int value_layout, "
@@ -461,6 +505,7 @@ TORCH_LIBRARY(sageattention, m) {
 
 TORCH_LIBRARY_IMPL(sageattention, CUDA, m) {
   m.impl("sageattn_fwd", &sageattn_fwd);
+  m.impl("sageattn_kv_fwd", &sageattn_kv_fwd);
   m.impl("qk_int8_sv_f16_attn", &qk_int8_sv_f16_attn);
   m.impl("fp16_attn", &fp16_attn);
   m.impl("bf16_attn", &bf16_attn);
@@ -473,7 +518,119 @@ TORCH_LIBRARY_IMPL(sageattention, CUDA, m) {
   m.impl("v_to_f16", &v_to_f16);
 }
 
-// An otherwise empty CPython module, so that `import sageattention_rdna3_b200._C` loads the
-// library and runs the registrations above (the reference does the same, csrc/pybind_gfx11.cpp:6-16).
-static struct PyModuleDef sage_module_def = {PyModuleDef_HEAD_INIT, "_C", nullptr, -1, nullptr};
+// ---------------------------------------------------------------- the module `_C`
+// Importing it runs the registrations above (the reference does the same, csrc/pybind_gfx11.cpp:6-16).
+// It also holds the short way into sageattn_fwd.  A small call is bound by the host: of 16-20 us per call
+// (1024 tokens and below), the checks of core.sageattn took 7 and the conversion of twelve arguments by
+// torch.ops another 3.  sageattn_plain makes the same checks on the tensors themselves, and calls the
+// same operator through the dispatcher; whatever is not a plain call - a check that fails, an argument of
+// another type, a tensor subclass or wrapper, an active mode, an environment variable that changes the
+// route - returns None and takes the way through core.py, which raises the errors.
+namespace {
+
+struct DeviceState {
+  at::Tensor status;           // the status word of core.py
+  at::Tensor mirror;           // its copy in pinned host memory; undefined if that is switched off
+};
+constexpr int kMaxDevices = 64;
+// Written by register_device and read by sageattn_plain, both with the GIL held.  Never freed: the
+// tensors must not be destroyed after the CUDA runtime at process exit.
+DeviceState* g_devices[kMaxDevices];
+
+bool env_set(const char* name) {
+  const char* e = std::getenv(name);                     // os.environ writes through to it
+  return e != nullptr && *e != '\0';
+}
+
+// The reference's dispatch (core.py use_direct_kernel) with its default thresholds.
+bool direct_by_default(int64_t D, int64_t layout, bool causal, int64_t q_len, int64_t kv_len) {
+  if (D == 64) {
+    if (causal || q_len < kv_len) return kv_len <= 6144;
+    return kv_len <= (layout == kHND ? 2048 : 3072);
+  }
+  return kv_len <= (q_len * 2 < kv_len ? 4096 : 2048);
+}
+
+bool aligned_16b(const at::Tensor& t) {
+  return t.stride(3) == 1 && ((t.stride(0) | t.stride(1) | t.stride(2)) & 7) == 0 &&
+         (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+}
+
+// register_device(index, status, mirror or None)
+PyObject* register_device(PyObject*, PyObject* args) {
+  HANDLE_TH_ERRORS
+  int idx = 0;
+  PyObject *status = nullptr, *mirror = nullptr;
+  if (!PyArg_ParseTuple(args, "iOO", &idx, &status, &mirror)) return nullptr;
+  TORCH_CHECK(idx >= 0 && THPVariable_Check(status) && (mirror == Py_None || THPVariable_Check(mirror)),
+              "register_device: bad argument");
+  if (idx < kMaxDevices && g_devices[idx] == nullptr) {
+    DeviceState* d = new DeviceState;
+    d->status = THPVariable_Unpack(status);
+    if (mirror != Py_None) d->mirror = THPVariable_Unpack(mirror);
+    g_devices[idx] = d;
+  }
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// sageattn_plain(q, k, v, tensor_layout, is_causal, sm_scale, smooth_k) -> Tensor or None
+PyObject* sageattn_plain(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 7 || !THPVariable_CheckExact(args[0]) || !THPVariable_CheckExact(args[1]) || !THPVariable_CheckExact(args[2]) ||
+      !PyUnicode_CheckExact(args[3]) || !PyBool_Check(args[4]) || (args[5] != Py_None && !PyFloat_CheckExact(args[5])) ||
+      !PyBool_Check(args[6]) || at::impl::torch_function_mode_enabled()) {
+    Py_RETURN_NONE;
+  }
+  const at::Tensor& q = THPVariable_Unpack(args[0]);
+  const at::Tensor& k = THPVariable_Unpack(args[1]);
+  const at::Tensor& v = THPVariable_Unpack(args[2]);
+  for (const at::Tensor* t : {&q, &k, &v}) {
+    if (at::isTensorSubclassLike(*t) || t->layout() != at::kStrided || !t->is_cuda() || t->dim() != 4) Py_RETURN_NONE;
+    if (t->unsafeGetTensorImpl()->has_symbolic_sizes_strides() || t->is_neg() || t->is_conj()) Py_RETURN_NONE;
+  }
+  int64_t layout = -1;
+  if (PyUnicode_CompareWithASCIIString(args[3], "HND") == 0) layout = kHND;
+  else if (PyUnicode_CompareWithASCIIString(args[3], "NHD") == 0) layout = kNHD;
+  const at::ScalarType dt = q.scalar_type();
+  if (layout < 0 || (dt != at::kHalf && dt != at::kBFloat16) || k.scalar_type() != dt || v.scalar_type() != dt ||
+      k.device() != q.device() || v.device() != q.device() || k.sizes() != v.sizes() || q.numel() == 0 || k.numel() == 0 ||
+      !aligned_16b(q) || !aligned_16b(k) || !aligned_16b(v)) {
+    Py_RETURN_NONE;
+  }
+  const Dims dq = dims_of(q, layout), dk = dims_of(k, layout);
+  if (dq.B != dk.B || dq.D != dk.D || (dq.D != 64 && dq.D != 128) || dq.H % dk.H != 0) Py_RETURN_NONE;
+  const int idx = q.get_device();
+  if (idx < 0 || idx >= kMaxDevices || g_devices[idx] == nullptr) Py_RETURN_NONE;   // the long way registers it
+  const DeviceState& dev = *g_devices[idx];
+  if (dev.mirror.defined() && *static_cast<volatile int32_t*>(dev.mirror.data_ptr()) != 0) Py_RETURN_NONE;
+  if (env_set("SAGEATTN_KERNEL") || env_set("SAGEATTN_B200_CHECK_STATUS") || env_set("SAGEATTN_DIRECT_THRESHOLD_D64") ||
+      env_set("SAGEATTN_DIRECT_THRESHOLD_D64_CAUSAL") || env_set("SAGEATTN_DIRECT_THRESHOLD_D64_CROSS") ||
+      env_set("SAGEATTN_DIRECT_THRESHOLD_D128") || env_set("SAGEATTN_DIRECT_THRESHOLD_D128_CROSS")) {
+    Py_RETURN_NONE;
+  }
+  const bool causal = args[4] == Py_True;
+  const bool direct = direct_by_default(dq.D, layout, causal, dq.S, dk.S);
+  const bool smooth = args[6] == Py_True && !direct;     // the un-quantised branch has no use for the mean
+  const double sm_scale = args[5] == Py_None ? std::pow(static_cast<double>(dq.D), -0.5) : PyFloat_AS_DOUBLE(args[5]);
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("sageattention::sageattn_fwd", "")
+                             .typed<decltype(sageattn_fwd)>();
+  at::Tensor out;
+  {
+    pybind11::gil_scoped_release no_gil;
+    out = op.call(q, k, v, layout, causal, sm_scale, smooth, direct, dev.status, c10::nullopt, c10::nullopt,
+                  at::OptionalIntArrayRef())[0];
+  }
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef sage_methods[] = {
+    {"register_device", register_device, METH_VARARGS, nullptr},
+    {"sageattn_plain", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(sageattn_plain)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+}  // namespace
+
+static struct PyModuleDef sage_module_def = {PyModuleDef_HEAD_INIT, "_C", nullptr, -1, sage_methods};
 PyMODINIT_FUNC PyInit__C(void) { return PyModule_Create(&sage_module_def); }

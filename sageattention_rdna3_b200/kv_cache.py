@@ -104,19 +104,10 @@ def sageattn_quantized_kv(q: torch.Tensor, kv: QuantizedKV, is_causal: bool = Fa
     if q.data_ptr() % 16 != 0:
         q = q.clone(memory_format=torch.contiguous_format)
     ops = _native.load_ops()
-    o = torch.empty_like(q)
+    if q.numel() > 0 and kv.k_int8.numel() > 0:
+        out = ops.sageattn_kv_fwd(q, kv.k_int8, kv.k_scale, kv.v16, kv.k_mean, layout, kv.v_layout, int(is_causal), sm_scale,
+                                  _status_word(q.device), int(return_lse))
+        return (out[0], out[1]) if return_lse else out[0]
+    o = torch.zeros_like(q)
     lse = torch.full((B, Hq, q_len), float("-inf"), dtype=torch.float32, device=q.device) if return_lse else None
-    if q_len == 0 or B == 0 or Hq == 0:
-        pass
-    elif kv.kv_len == 0:
-        o.zero_()
-    else:
-        shape = list(q.shape)
-        shape[seq_dim], shape[head_idx] = 0, kv.num_kv_heads
-        no_k = q.new_empty(shape)           # an empty key: only the Q blocks of the launch exist
-        q_int8, q_scale, _, _ = ops.quant_qk_int8(q, no_k, q.new_empty(0), layout, sm_scale)
-        ops.qk_int8_sv_f16_attn(q_int8, kv.k_int8, kv.v16, o, q_scale, kv.k_scale, layout, int(is_causal), sm_scale,
-                                value_layout=kv.v_layout, status=_status_word(q.device), lse=lse)
-        if return_lse and kv.k_mean is not None:
-            ops.lse_add_q_mean(lse, q, kv.k_mean, layout, sm_scale)
     return (o, lse) if return_lse else o
