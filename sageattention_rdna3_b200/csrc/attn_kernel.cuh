@@ -268,6 +268,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int lane = threadIdx.x & 31;
 
   if ((smem_u32(smem) & 1023u) != 0u) {        // swizzled tiles need 1024-byte alignment
+    grid_dependency_wait();
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, kStatusSmemMisaligned);
     return;
   }
@@ -292,13 +293,6 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 4);
   int* fail_code = reinterpret_cast<int*>(smem + L::kOffMisc + 8);
 
-  if (threadIdx.x == 0) {
-    // A status word that is already set means an earlier CTA of this launch (or an earlier launch
-    // the caller has not looked at yet) gave up: this CTA leaves through the abort path at once, so a
-    // failing launch costs about one wait bound and not one per wave of CTAs.
-    *abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
-    *fail_code = 0;
-  }
   // TMA loads of the producer thread.  int8 Q / K are contiguous [B*H, S, D] (3-D maps); 16-bit Q / K
   // come in the caller's layout, one [128 rows][64 columns] box per 64 columns of head_dim.
   auto load_q = [&](const Segment& g) {
@@ -319,10 +313,8 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       tma_load_3d(s_k + stage * L::kKBytes, &tm_k, k_full + stage, 0, tile * kBlockN, g.b * p.Hkv + g.hkv);
     }
   };
+  // Set-up that touches no global memory runs under the end of the kernel ahead in the stream.
   if (warp == 4 && elect_one()) {
-    // The producer thread sets the barriers up itself and starts the first loads (Q and K tile 0,
-    // which wait for nothing) at once, so their latency overlaps the TMEM allocation and the
-    // CTA-wide barrier below.
     mbar_init(q_full, 1);
     mbar_init(o_final, 1);
     mbar_init(q_empty, 1);
@@ -345,6 +337,25 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
     tma_prefetch_desc(&tm_o);
+  }
+  if (warp == 5) {
+    tmem_alloc(tmem_slot, kTmemCols);
+    tmem_relinquish();
+  }
+  grid_dependency_wait();
+  // Only the persistent launch lets the next kernel (its merge) start early: blocks of a following
+  // preparation that wait beside the tail of a plain launch cost more than they gain (B=2 H=32 S=8192
+  // causal: 983 us per call with it, 937 without).
+  if (STREAMK) grid_launch_dependents();
+  if (threadIdx.x == 0) {
+    // A status word that is already set means an earlier CTA of this launch (or an earlier launch
+    // the caller has not looked at yet) gave up: this CTA leaves through the abort path at once, so a
+    // failing launch costs about one wait bound and not one per wave of CTAs.
+    *abort_flag = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    *fail_code = 0;
+  }
+  if (warp == 4 && elect_one()) {        // the same thread as above: elect.sync is deterministic
+    // The first loads (Q and K tile 0) wait for nothing in this CTA: their latency overlaps the barrier below.
     SegIter<CAUSAL, STREAMK> first_iter(p);
     Segment g0;
     if (first_iter.next(g0) && g0.n_kv > 0) {
@@ -353,10 +364,6 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       mbar_arrive_expect_tx(k_full, L::kKBytes);
       load_k(g0, g0.kv_lo, 0);
     }
-  }
-  if (warp == 5) {
-    tmem_alloc(tmem_slot, kTmemCols);
-    tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
@@ -907,6 +914,8 @@ template <int D>
 __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams p) {
   __shared__ float row_max[kMergeRows];
   __shared__ float row_inv[kMergeRows];
+  grid_dependency_wait();
+  grid_launch_dependents();
   const int item = blockIdx.x / kMergeSplit;
   const int row0 = (blockIdx.x - item * kMergeSplit) * kMergeRows;     // first row of this CTA within the item
   const int bh = item / p.n_q_tiles;

@@ -102,6 +102,8 @@ __global__ void __launch_bounds__(256) sage_lse_mean_kernel(const StridedView q,
                                                             float* __restrict__ lse, int Hq, int rep, int Sq,
                                                             long long rows, float sm_scale) {
   constexpr int kLanes = D / 8;
+  grid_dependency_wait();
+  grid_launch_dependents();
   const long long idx = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   const long long row = idx / kLanes;
   const int c = static_cast<int>(idx % kLanes) * 8;

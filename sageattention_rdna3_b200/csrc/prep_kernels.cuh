@@ -316,6 +316,8 @@ __device__ __forceinline__ void prep_v_block(const PrepParams& p, int blk) {
 template <typename T, int D>
 __global__ void __launch_bounds__(kPrepThreads, 4) sage_prep_kernel(const PrepParams p) {
   __shared__ float warp_max[kPrepWarps];
+  grid_dependency_wait();
+  grid_launch_dependents();
   int blk = blockIdx.x;
   if (blk < p.q_blocks) {
     prep_q_block<T, D, kPrepThreads>(p, blk, warp_max);
@@ -375,6 +377,8 @@ __global__ void __cluster_dims__(kMeanCluster, 1, 1) __launch_bounds__(256) sage
   constexpr int kOwnCols = D / kMeanCluster;                // columns this CTA sums in the end
   static_assert(kSets >= 1 && kOwnCols % 8 == 0, "tile shape");
   __shared__ __align__(16) float part[kMeanPartials][kOwnCols];
+  grid_dependency_wait();
+  grid_launch_dependents();
 
   const int tid = threadIdx.x;
   const uint32_t rank = blockIdx.x;                         // cluster = the 8 CTAs of one blockIdx.(y,z)
@@ -473,6 +477,8 @@ sage_prep_smooth_kernel(const PrepParams p) {
   constexpr int kOwnCols = D / kMeanCluster;
   static_assert(kActive <= kFusedThreads && kOwnCols % 8 == 0, "tile shape");
   __shared__ __align__(16) float part[kMeanPartials][kOwnCols];
+  grid_dependency_wait();
+  grid_launch_dependents();
   __shared__ __align__(16) T mean_s[D];
   __shared__ float warp_max[kFusedThreads / 32];
 

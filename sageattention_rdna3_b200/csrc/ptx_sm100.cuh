@@ -21,6 +21,16 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// ---------------------------------------------------------------- launch overlap ---------------
+// A kernel launched with programmatic serialisation may start before the kernel ahead of it in the
+// stream has ended: `grid_dependency_wait` returns when that one has completed and its writes are
+// visible; only what touches no global memory may come before it.  `grid_launch_dependents` lets the
+// next kernel start.  It is called AFTER the wait, so that no more than two kernels of a stream overlap
+// and the first level cache of an SM cannot hold lines that an older kernel read and the kernel ahead
+// overwrites.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // True in one thread of the (converged) warp.  tcgen05.mma, tcgen05.commit and the TMA instructions take
 // their operands from uniform registers: inside a branch on elect.sync the compiler knows that one
 // thread is active and moves them over directly; behind `lane == 0` it emits a loop over the active

@@ -115,13 +115,34 @@ int encode_strided_16bit(CUtensorMap* map, CUtensorMapDataType dt, const void* b
   return encode_map(map, dt, 4, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, what);
 }
 
+// Launch with programmatic serialisation: the set-up of the kernel and its launch latency run under the end
+// of the kernel ahead of it in the stream (every kernel launched here begins with
+// grid_dependency_wait()).  A call is one to four kernels, most of them short.  Calls back to back, before
+// and after: 20 heads of 1024 tokens, D=64 19.4 -> 17.3 us, 10 heads of 4096 tokens 85.4 -> 81.3, 32 heads
+// of 4096 tokens causal, D=128 161 -> 154, B=2 H=32 S=8192 causal 944 -> 937.
+template <typename... Params, typename... Args>
+int launch(void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchAttribute attr;
+  memset(&attr, 0, sizeof(attr));
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  SAGE_CUDA(cudaLaunchKernelEx(&cfg, kern, Params(args)...));
+  return SAGE_OK;
+}
+
 template <typename T, int D>
 int launch_prep(const sage::PrepParams& p, int v_blocks, cudaStream_t stream) {
   const int grid = p.q_blocks + p.k_blocks + v_blocks;
   if (grid == 0) return SAGE_OK;
-  sage::sage_prep_kernel<T, D><<<grid, sage::kPrepThreads, 0, stream>>>(p);
-  SAGE_CUDA(cudaGetLastError());
-  return SAGE_OK;
+  return launch(sage::sage_prep_kernel<T, D>, grid, sage::kPrepThreads, 0, stream, p);
 }
 
 int dispatch_prep(int dtype, int D, const sage::PrepParams& p, int v_blocks, cudaStream_t stream) {
@@ -290,9 +311,7 @@ int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
   if (rc) return rc;
   const long long grid = static_cast<long long>(p.n_q_tiles) * p.B * p.Hq;
   if (grid > 0x7fffffffLL) return fail(SAGE_ERR_INVALID, "too many query tiles for one launch (%lld)", grid);
-  kern<<<static_cast<unsigned>(grid), sage::kAttnThreads, kSmem, stream>>>(tq, tk, tv, to, p);
-  SAGE_CUDA(cudaGetLastError());
-  return SAGE_OK;
+  return launch(kern, static_cast<unsigned>(grid), sage::kAttnThreads, kSmem, stream, tq, tk, tv, to, p);
 }
 
 // The persistent launch and its merge.  `workspace` holds the partial results:
@@ -310,8 +329,8 @@ int launch_attn_streamk(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   p.sk_nkv_full = plan.nkv_full;
   p.part_o = static_cast<float*>(workspace);
   p.part_lse = p.part_o + static_cast<size_t>(plan.grid) * 2 * sage::kBlockM * D;
-  kern<<<static_cast<unsigned>(plan.grid), sage::kAttnThreads, kSmem, stream>>>(tq, tk, tv, to, p);
-  SAGE_CUDA(cudaGetLastError());
+  rc = launch(kern, static_cast<unsigned>(plan.grid), sage::kAttnThreads, kSmem, stream, tq, tk, tv, to, p);
+  if (rc) return rc;
   sage::MergeParams m;
   m.part_o = p.part_o; m.part_lse = p.part_lse;
   m.o = p.o; m.o_stride_b = p.o_stride_b; m.o_stride_h = p.o_stride_h; m.o_stride_s = p.o_stride_s;
@@ -321,9 +340,7 @@ int launch_attn_streamk(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   m.attn_grid = plan.grid;
   m.causal = CAUSAL ? 1 : 0; m.out_bf16 = p.out_bf16;
   const long long items = static_cast<long long>(p.n_q_tiles) * p.B * p.Hq;
-  sage::sage_attn_merge_kernel<D><<<static_cast<unsigned>(items * sage::kMergeSplit), 256, 0, stream>>>(m);
-  SAGE_CUDA(cudaGetLastError());
-  return SAGE_OK;
+  return launch(sage::sage_attn_merge_kernel<D>, static_cast<unsigned>(items * sage::kMergeSplit), 256, 0, stream, m);
 }
 
 // Device address of g_static_kmean on the current device, looked up once per device.
@@ -386,14 +403,10 @@ int sage_mean_seq(const sage_strided_t* k, int dtype, int B, int H, int S, int D
   dim3 grid(sage::kMeanCluster, H, B);                  // one cluster of 8 CTAs per (b, h)
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == SAGE_DTYPE_F16) {
-    if (D == 128) sage::sage_kmean_kernel<__half, 128><<<grid, 256, 0, st>>>(p);
-    else sage::sage_kmean_kernel<__half, 64><<<grid, 256, 0, st>>>(p);
-  } else {
-    if (D == 128) sage::sage_kmean_kernel<__nv_bfloat16, 128><<<grid, 256, 0, st>>>(p);
-    else sage::sage_kmean_kernel<__nv_bfloat16, 64><<<grid, 256, 0, st>>>(p);
+    return launch(D == 128 ? sage::sage_kmean_kernel<__half, 128> : sage::sage_kmean_kernel<__half, 64>, grid, 256, 0, st, p);
   }
-  SAGE_CUDA(cudaGetLastError());
-  return SAGE_OK;
+  return launch(D == 128 ? sage::sage_kmean_kernel<__nv_bfloat16, 128> : sage::sage_kmean_kernel<__nv_bfloat16, 64>, grid, 256,
+                0, st, p);
 }
 
 int sage_quant_qk_int8(const sage_strided_t* q, const sage_strided_t* k, const void* k_mean,
@@ -503,14 +516,11 @@ int sage_prep_smooth_qkv(const sage_strided_t* q, const sage_strided_t* k, const
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned g = static_cast<unsigned>(grid);
   if (dtype == SAGE_DTYPE_F16) {
-    if (D == 128) sage::sage_prep_smooth_kernel<__half, 128><<<g, sage::kFusedThreads, 0, st>>>(p);
-    else sage::sage_prep_smooth_kernel<__half, 64><<<g, sage::kFusedThreads, 0, st>>>(p);
-  } else {
-    if (D == 128) sage::sage_prep_smooth_kernel<__nv_bfloat16, 128><<<g, sage::kFusedThreads, 0, st>>>(p);
-    else sage::sage_prep_smooth_kernel<__nv_bfloat16, 64><<<g, sage::kFusedThreads, 0, st>>>(p);
+    return launch(D == 128 ? sage::sage_prep_smooth_kernel<__half, 128> : sage::sage_prep_smooth_kernel<__half, 64>, g,
+                  sage::kFusedThreads, 0, st, p);
   }
-  SAGE_CUDA(cudaGetLastError());
-  return SAGE_OK;
+  return launch(D == 128 ? sage::sage_prep_smooth_kernel<__nv_bfloat16, 128> : sage::sage_prep_smooth_kernel<__nv_bfloat16, 64>,
+                g, sage::kFusedThreads, 0, st, p);
 }
 
 int sage_quant_qk_int8_smooth_static(const sage_strided_t* q, const sage_strided_t* k, int dtype, int B, int Hq,
@@ -780,16 +790,11 @@ int sage_lse_add_q_mean(const sage_strided_t* q, int dtype, const void* k_mean, 
   const sage::StridedView v = view_of(q);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define SAGE_LSE_MEAN(T, DD)                                                                                   \
-  sage::sage_lse_mean_kernel<T, DD><<<static_cast<unsigned>(blocks), 256, 0, st>>>(v, static_cast<const T*>(k_mean), lse, Hq, \
-                                                                                   Hq / Hkv, Sq, rows, sm_scale)
-  if (dtype == SAGE_DTYPE_BF16) {
-    if (D == 128) SAGE_LSE_MEAN(__nv_bfloat16, 128); else SAGE_LSE_MEAN(__nv_bfloat16, 64);
-  } else {
-    if (D == 128) SAGE_LSE_MEAN(__half, 128); else SAGE_LSE_MEAN(__half, 64);
-  }
+  launch(sage::sage_lse_mean_kernel<T, DD>, static_cast<unsigned>(blocks), 256, 0, st, v, static_cast<const T*>(k_mean), lse, \
+         Hq, Hq / Hkv, Sq, rows, sm_scale)
+  if (dtype == SAGE_DTYPE_BF16) return D == 128 ? SAGE_LSE_MEAN(__nv_bfloat16, 128) : SAGE_LSE_MEAN(__nv_bfloat16, 64);
+  return D == 128 ? SAGE_LSE_MEAN(__half, 128) : SAGE_LSE_MEAN(__half, 64);
 #undef SAGE_LSE_MEAN
-  SAGE_CUDA(cudaGetLastError());
-  return SAGE_OK;
 }
 
 int sage_fold_attn_partial(const sage_strided_t* o_acc, float* lse_acc, int64_t lse_stride_b, int64_t lse_stride_h,
