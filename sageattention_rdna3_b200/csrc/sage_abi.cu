@@ -314,6 +314,10 @@ int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
   return launch(kern, static_cast<unsigned>(grid), sage::kAttnThreads, kSmem, stream, tq, tk, tv, to, p);
 }
 
+// Up to this many items the merge takes the fewest rows per block (see sage_attn_merge_kernel): 128 items
+// are 512 blocks of 32 rows, less than one round of the 8 per SM.
+constexpr long long kFewMergeItems = 128;
+
 // The persistent launch and its merge.  `workspace` holds the partial results:
 // [grid][2][128][D] fp32 outputs, then [grid][2][128] fp32 log-sum-exps.
 template <int D, bool CAUSAL, bool QKF>
@@ -340,7 +344,12 @@ int launch_attn_streamk(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   m.attn_grid = plan.grid;
   m.causal = CAUSAL ? 1 : 0; m.out_bf16 = p.out_bf16;
   const long long items = static_cast<long long>(p.n_q_tiles) * p.B * p.Hq;
-  return launch(sage::sage_attn_merge_kernel<D>, static_cast<unsigned>(items * sage::kMergeSplit), 256, 0, stream, m);
+  constexpr int kFew = sage::merge_rows_few(D);
+  if (items <= kFewMergeItems) {
+    return launch(sage::sage_attn_merge_kernel<D, kFew>, static_cast<unsigned>(items * (sage::kBlockM / kFew)), 256, 0, stream, m);
+  }
+  return launch(sage::sage_attn_merge_kernel<D, sage::kMergeRows>,
+                static_cast<unsigned>(items * (sage::kBlockM / sage::kMergeRows)), 256, 0, stream, m);
 }
 
 // Device address of g_static_kmean on the current device, looked up once per device.
