@@ -690,7 +690,9 @@ int attn_int8_impl(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t*
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (Sq == 0) return SAGE_OK;
 
-  const int fold = (s_dump == nullptr && n_peers == 0) ? sage_gqa_fold(Hq, Hkv, Sq, o_stride_h, o_stride_s, is_causal) : 1;
+  // (Scattering launches fold as well: the copies have the strides of `o`, and each must equal the plain
+  // launch's result bit for bit.)
+  const int fold = (s_dump == nullptr) ? sage_gqa_fold(Hq, Hkv, Sq, o_stride_h, o_stride_s, is_causal) : 1;
   const int rows_per_head = Sq;
   if (fold > 1) {
     Hq /= fold;

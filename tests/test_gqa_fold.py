@@ -83,3 +83,33 @@ def test_fold_rule_on_the_host(tmp_path):
             assert fold(hq, hkv, sq, 128, hq * 128, 0) == (rep if fewer and sq * hq == 1 else 1)   # NHD
             assert fold(hq, hkv, sq, sq * 128 + 8, 128, 0) == 1                  # padded heads
     assert fold(4, 0, 8, 8, 1, 0) == 1 and fold(4, 2, 0, 0, 1, 0) == 1 and fold(5, 2, 8, 8, 1, 0) == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,Hkv,rep,Sq,Skv,D,dtype", [
+    (2, 2, 4, 1, 300, 128, torch.bfloat16),
+    (1, 2, 4, 31, 257, 128, torch.float16),       # the rows of a warp belong to two heads
+    (2, 1, 8, 33, 129, 64, torch.bfloat16),
+    (1, 2, 2, 160, 513, 64, torch.float16),
+])
+def test_scattering_launch_folds_like_the_plain_one(B, Hkv, rep, Sq, Skv, D, dtype):
+    """Every copy that a scattering launch writes equals the result of the plain launch bit for bit, also where
+    that one folds the heads (which rows share a warp decides when a running maximum moves, and with it the
+    rounding of P).  Keys that grow along the sequence make the maxima move."""
+    from sageattention_rdna3_b200 import check_status, sageattn
+    g = torch.Generator(device="cpu").manual_seed(Sq + D)
+    q = (torch.randn(B, Hkv * rep, Sq, D, generator=g) * 4).to(dtype).cuda()
+    k = (torch.randn(B, Hkv, Skv, D, generator=g) * torch.linspace(0.5, 4.0, Skv)[:, None]).to(dtype).cuda()
+    v = torch.randn(B, Hkv, Skv, D, generator=g).to(dtype).cuda()
+    try:
+        H.set_streamk(0)
+        want = sageattn(q, k, v, kernel="int8")
+        out = torch.empty_like(q)
+        copies = [torch.full_like(q, float("nan")) for _ in range(3)]
+        got = sageattn(q, k, v, kernel="int8", out=out, scatter_to=[c.data_ptr() for c in copies])
+    finally:
+        H.set_streamk(-1)
+    check_status()
+    assert torch.equal(got, want)
+    for c in copies:
+        assert torch.equal(c, want)
