@@ -151,7 +151,8 @@ constexpr int kHalfN = kBlockN / 2;      // the softmax works on 64-column halve
 #ifndef SAGE_DEPHASE
 #define SAGE_DEPHASE 1
 #endif
-static __device__ unsigned g_sm_arrivals[1024];
+constexpr int kMaxSmIds = 1024;
+static __device__ unsigned g_sm_arrivals[kMaxSmIds];
 
 // What one pass of the pipeline works on: KV tiles [kv_lo, kv_lo + n_kv) of one 128-row query tile
 // of one (batch, query head).  slot < 0: the pass covers every KV tile of the item and writes the
@@ -313,7 +314,8 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       tma_load_3d(s_k + stage * L::kKBytes, &tm_k, k_full + stage, 0, tile * kBlockN, g.b * p.Hkv + g.hkv);
     }
   };
-  // Set-up that touches no global memory runs under the end of the kernel ahead in the stream.
+  // Set-up that touches no global memory and takes nothing that the kernel ahead in the stream may still need
+  // runs under the end of that kernel.
   if (warp == 4 && elect_one()) {
     mbar_init(q_full, 1);
     mbar_init(o_final, 1);
@@ -338,11 +340,19 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     tma_prefetch_desc(&tm_v);
     tma_prefetch_desc(&tm_o);
   }
+  grid_dependency_wait();
+  // TMEM is taken after the wait.  The kernel ahead may be anybody's, and one that lets its successor start
+  // before it has allocated its own columns would find them held by CTAs that wait for it to end.
+  // The placement of CTAs that start early depends on it as well (recorded with %smid, 128 items behind their
+  // preparation): with the allocation before the wait 18 of 110 SMs got two CTAs and 38 none, after it
+  // every CTA has an SM to itself, as on an idle GPU.  4 heads of 4096 tokens, D=128: 62.1 -> 48.9 us per
+  // call; 6 heads of 3072, un-quantised, D=64: 44.4 -> 33.0.  Causal launches of some 400-1000 items had
+  // gained from the uneven placement, which is given up: 16 heads of 4096 tokens 82.8 -> 90.1 us (97 with
+  // ordinary launches).
   if (warp == 5) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
-  grid_dependency_wait();
   // Only the persistent launch lets the next kernel (its merge) start early: blocks of a following
   // preparation that wait beside the tail of a plain launch cost more than they gain (B=2 H=32 S=8192
   // causal: 983 us per call with it, 937 without).
@@ -560,7 +570,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (threadIdx.x == 0) {
         unsigned smid;
         asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-        *arrival = atomicAdd(&g_sm_arrivals[smid & 1023u], 1u);
+        *arrival = atomicAdd(&g_sm_arrivals[smid & (kMaxSmIds - 1)], 1u);
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");      // the four softmax warps only
       yields = (*arrival & 1u) != 0u;

@@ -25,4 +25,7 @@ extern "C" {
 // contiguous [B,Hkv,D] in the dtype of q.
 int sage_lse_add_q_mean(const sage_strided_t* q, int dtype, const void* k_mean, float* lse, int B, int Hq, int Hkv, int Sq,
                         int D, float sm_scale, void* stream);
+// Test hook: how many CTAs of plain attention launches have started on each SM of the current device (counted
+// since the library was loaded; synchronises).
+int sage_test_sm_arrivals(unsigned* counts, int n);
 }

@@ -393,6 +393,11 @@ int sage_set_streamk(int mode) {
   g_streamk_mode.store(mode, std::memory_order_relaxed);
   return SAGE_OK;
 }
+int sage_test_sm_arrivals(unsigned* counts, int n) {
+  SAGE_REQUIRE(counts != nullptr && n > 0 && n <= sage::kMaxSmIds, "sage_test_sm_arrivals: bad argument");
+  SAGE_CUDA(cudaMemcpyFromSymbol(counts, sage::g_sm_arrivals, static_cast<size_t>(n) * sizeof(unsigned)));
+  return SAGE_OK;
+}
 int sage_test_drop_v_load(int on) {
   g_test_drop_v_load.store(on ? 1 : 0, std::memory_order_relaxed);
   return SAGE_OK;

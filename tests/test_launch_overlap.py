@@ -27,3 +27,58 @@ def test_back_to_back_calls_on_buffers_that_change(D, S, smooth, dtype):
     torch.cuda.synchronize()
     assert all(torch.equal(o, want[i % 4]) for i, o in enumerate(got))
     assert all(torch.equal(o, chained[0]) for o in chained)
+
+
+def test_nothing_shared_is_taken_before_the_kernel_ahead_has_ended():
+    """Read from the source (a kernel that breaks this may wait for ever, so it is not run): in the attention
+    kernel nothing before the first dependency wait of the normal path allocates TMEM, starts a copy or reads
+    global memory through the parameters."""
+    import re
+    from sageattention_rdna3_b200.build import CSRC
+    text = re.sub(r"//[^\n]*", "", (CSRC / "attn_kernel.cuh").read_text())
+    body = text[text.index("\nsage_attn_kernel("):]
+    setup = body.index("mbar_init(q_full")
+    before = body[setup:body.index("grid_dependency_wait();", setup)]
+    for word in ("tmem_alloc", "load_q(", "load_k(", "tma_load", "p.status", "p.q_scale", "__ldg", "atomic"):
+        assert word not in before, word
+    assert body.index("tmem_alloc(") > body.index("grid_dependency_wait();", setup)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,S,D,dtype,kernel,smooth", [
+    (4, 4096, 128, torch.bfloat16, "int8", False), (8, 2304, 128, torch.bfloat16, "int8", True),
+    (4, 4500, 64, torch.float16, "int8", False), (8, 2048, 64, torch.bfloat16, "direct", False),
+    (6, 3072, 64, torch.bfloat16, "direct", False)])
+def test_small_launches_get_an_sm_per_block(H, S, D, dtype, kernel, smooth):
+    """128 to 144 plain attention blocks behind a preparation that lets them start early: no SM runs two of them
+    while others run none (counted by the kernel itself)."""
+    import ctypes
+    import helpers
+    from sageattention_rdna3_b200 import _native, sageattn
+    lib = _native.load_abi()
+    n_sms = torch.cuda.get_device_properties(0).multi_processor_count
+    items = H * -(-S // 128)
+    if items > n_sms:
+        pytest.skip("needs an SM for every block")
+
+    def counts():
+        c = (ctypes.c_uint32 * 1024)()
+        assert lib.sage_test_sm_arrivals(c, 1024) == 0
+        return list(c)
+
+    torch.manual_seed(0)
+    q, k, v = (torch.randn(1, S, H, D, device="cuda").to(dtype) for _ in range(3))
+    call = lambda: sageattn(q, k, v, tensor_layout="NHD", kernel=kernel, smooth_k=smooth)
+    try:
+        helpers.set_streamk(0)
+        call()
+        for _ in range(4):
+            torch.cuda.synchronize()
+            before = counts()
+            torch.cuda._sleep(1_000_000)         # about half a millisecond: both launches are queued before either runs
+            call()
+            torch.cuda.synchronize()
+            new = [b - a for a, b in zip(before, counts())]
+            assert sum(new) == items and max(new) == 1
+    finally:
+        helpers.set_streamk(-1)
