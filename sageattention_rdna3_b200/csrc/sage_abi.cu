@@ -42,10 +42,15 @@ int fail(int code, const char* fmt, ...) {
     if (!(cond)) return fail(SAGE_ERR_INVALID, __VA_ARGS__); \
   } while (0)
 
-#define SAGE_CUDA(expr)                                                                        \
-  do {                                                                                         \
-    cudaError_t e_ = (expr);                                                                   \
-    if (e_ != cudaSuccess) return fail(SAGE_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(e_)); \
+// (The runtime keeps the error for the thread's next cudaGetLastError as well; it is taken from there, or the
+// caller's next launch of something else would report it a second time.)
+#define SAGE_CUDA(expr)                                                           \
+  do {                                                                            \
+    cudaError_t e_ = (expr);                                                      \
+    if (e_ != cudaSuccess) {                                                      \
+      cudaGetLastError();                                                         \
+      return fail(SAGE_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(e_));        \
+    }                                                                             \
   } while (0)
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
