@@ -135,9 +135,12 @@ int sage_qk_int8_sv_f16_attn_lse(const int8_t* q_i8, const int8_t* k_i8, const s
  * kernel; they fall back to the plain launch when that would not pay, when the workspace is NULL
  * or too small, or when s_dump is set.  Results agree with the plain launch to fp32 rounding of
  * the merge (same int8 products, same softmax).
- * sage_attn_workspace_bytes: bytes the _ws calls want for this problem on the current device, 0 if
- * they would use the plain launch anyway.  The workspace needs no initialisation and may be
- * reused by the next call on the same stream. */
+ * The INT8 launch lets the query heads of a GQA group share query tiles where that gives fewer of them
+ * (few queries per head, no causal mask, no s_dump, output rows that run on from one head to the next:
+ * o_stride_h == Sq * o_stride_s), and cuts up the tiles that result.
+ * sage_attn_workspace_bytes: the most that a _ws call with these sizes takes on the current device, whatever
+ * its number of kv heads and its output strides; 0 if all of them would use the plain launch anyway.  The
+ * workspace needs no initialisation and may be reused by the next call on the same stream. */
 int64_t sage_attn_workspace_bytes(int B, int Hq, int Sq, int Skv, int D, int is_causal);
 int sage_qk_int8_sv_f16_attn_ws(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t* v16, void* o,
                                 int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_s, const float* q_scale,

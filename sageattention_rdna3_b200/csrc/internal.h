@@ -25,6 +25,12 @@ extern "C" {
 // contiguous [B,Hkv,D] in the dtype of q.
 int sage_lse_add_q_mean(const sage_strided_t* q, int dtype, const void* k_mean, float* lse, int B, int Hq, int Hkv, int Sq,
                         int D, float sm_scale, void* stream);
+// Workspace bytes of one launch, as it will plan it: of sage_qk_int8_sv_f16_attn_ws with these sizes and output
+// strides (heads folded where the rule above says so), and of sage_direct_attn_ws.  The public
+// sage_attn_workspace_bytes knows neither the kv heads nor the strides and gives the most that any of them takes.
+int64_t sage_int8_workspace_bytes(int B, int Hq, int Hkv, int Sq, int Skv, int D, int is_causal, int64_t o_stride_h,
+                                  int64_t o_stride_s);
+int64_t sage_direct_workspace_bytes(int B, int Hq, int Sq, int Skv, int D, int is_causal);
 // Test hook: how many CTAs of plain attention launches have started on each SM of the current device (counted
 // since the library was loaded; synchronises).
 int sage_test_sm_arrivals(unsigned* counts, int n);

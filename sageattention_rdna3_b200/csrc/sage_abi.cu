@@ -592,11 +592,25 @@ int sage_qk_int8_sv_f16_attn_lse(const int8_t* q_i8, const int8_t* k_i8, const s
                                      stream);
 }
 
-int64_t sage_attn_workspace_bytes(int B, int Hq, int Sq, int Skv, int D, int is_causal) {
+int64_t sage_direct_workspace_bytes(int B, int Hq, int Sq, int Skv, int D, int is_causal) {
   StreamKPlan plan;
   if (B <= 0 || Hq <= 0 || (D != 64 && D != 128)) return 0;
   if (plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal) != SAGE_OK) return 0;
   return plan.use ? static_cast<int64_t>(plan.workspace_bytes) : 0;
+}
+
+int64_t sage_int8_workspace_bytes(int B, int Hq, int Hkv, int Sq, int Skv, int D, int is_causal, int64_t o_stride_h,
+                                  int64_t o_stride_s) {
+  const int fold = sage_gqa_fold(Hq, Hkv, Sq, o_stride_h, o_stride_s, is_causal);
+  return sage_direct_workspace_bytes(B, Hq / fold, Sq * fold, Skv, D, is_causal);
+}
+
+int64_t sage_attn_workspace_bytes(int B, int Hq, int Sq, int Skv, int D, int is_causal) {
+  int64_t most = sage_direct_workspace_bytes(B, Hq, Sq, Skv, D, is_causal);
+  for (int hkv = 1; hkv < Hq; ++hkv) {                   // the numbers of kv heads for which heads would be folded
+    if (Hq % hkv == 0) most = std::max(most, sage_int8_workspace_bytes(B, Hq, hkv, Sq, Skv, D, is_causal, Sq, 1));
+  }
+  return most;
 }
 
 namespace {

@@ -270,9 +270,8 @@ at::Tensor qk_int8_sv_f16_attn(const at::Tensor& q_i8, const at::Tensor& k_i8, c
   }
   // Problems that would fill the GPU unevenly run on persistent CTAs and need scratch for partial results.
   at::Tensor workspace;
-  const int64_t fold = sage_gqa_fold(Hq, Hkv, Sq, os.stride_h, os.stride_s, is_causal);   // as the launcher does
-  const int64_t ws_bytes =
-      dump_ptr ? 0 : sage_attn_workspace_bytes((int)B, (int)(Hq / fold), (int)(Sq * fold), (int)Skv, (int)D, (int)is_causal);
+  const int64_t ws_bytes = dump_ptr ? 0 : sage_int8_workspace_bytes((int)B, (int)Hq, (int)Hkv, (int)Sq, (int)Skv, (int)D,
+                                                                    (int)is_causal, os.stride_h, os.stride_s);
   if (ws_bytes > 0) workspace = at::empty({ws_bytes}, q_i8.options().dtype(at::kByte));
   check_rc(sage_qk_int8_sv_f16_attn_ws(q_i8.data_ptr<int8_t>(), k_i8.data_ptr<int8_t>(), &vs, o.data_ptr(), os.stride_b,
                                        os.stride_h, os.stride_s, q_scale.data_ptr<float>(),
@@ -332,7 +331,7 @@ at::Tensor direct_attn(const at::Tensor& q, const at::Tensor& k, const at::Tenso
     return o;
   }
   at::Tensor workspace;
-  const int64_t ws_bytes = sage_attn_workspace_bytes((int)dq.B, (int)dq.H, (int)dq.S, (int)dk.S, (int)dq.D, (int)is_causal);
+  const int64_t ws_bytes = sage_direct_workspace_bytes((int)dq.B, (int)dq.H, (int)dq.S, (int)dk.S, (int)dq.D, (int)is_causal);
   if (ws_bytes > 0) workspace = at::empty({ws_bytes}, q.options().dtype(at::kByte));
   check_rc(sage_direct_attn_ws(&qs, &ks, &vs, o.data_ptr(), os.stride_b, os.stride_h, os.stride_s, dtype_code(q),
                                (int)dq.B, (int)dq.H, (int)dk.H, (int)dq.S, (int)dk.S, (int)dq.D, (int)is_causal,

@@ -113,3 +113,30 @@ def test_scattering_launch_folds_like_the_plain_one(B, Hkv, rep, Sq, Skv, D, dty
     assert torch.equal(got, want)
     for c in copies:
         assert torch.equal(c, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv,D", [
+    (8, 32, 8, 64, 8192, 128),       # 256 tiles, which stay on the plain launch; folded 128, which do not
+    (4, 32, 8, 64, 8192, 128),       # persistent either way
+])
+def test_workspace_that_the_query_asks_for_is_used(B, Hq, Hkv, Sq, Skv, D):
+    """A caller of the C ABI that allocates what sage_attn_workspace_bytes says gets the launch that the operator
+    takes: it writes partial results to the workspace, and the output is the same bit for bit."""
+    from sageattention_rdna3_b200 import _native
+    lib, ops = _native.load_abi(), _native.load_ops()
+    H.set_streamk(-1)
+    q, k = H.randn((B, Hq, Sq, D), 0, torch.float16).cuda(), H.randn((B, Hkv, Skv, D), 1, torch.float16).cuda()
+    v = H.randn((B, Hkv, Skv, D), 2, torch.float16).cuda()
+    q_i8, q_scale, k_i8, k_scale, _ = H.abi_quant(q, k, None, "HND", D ** -0.5)
+    want = ops.qk_int8_sv_f16_attn(q_i8, k_i8, v, torch.empty_like(q), q_scale, k_scale, 1, 0, 1.0)
+    n = lib.sage_attn_workspace_bytes(B, Hq, Sq, Skv, D, 0)
+    assert n > 0
+    ws = torch.full((n // 4,), float("nan"), device="cuda")
+    o, vs = torch.empty_like(q), H.strided(v, "HND")
+    H._check(lib.sage_qk_int8_sv_f16_attn_ws(q_i8.data_ptr(), k_i8.data_ptr(), ctypes.byref(vs), o.data_ptr(), Hq * Sq * D,
+                                             Sq * D, D, q_scale.data_ptr(), k_scale.data_ptr(), 0, B, Hq, Hkv, Sq, Skv, D, 0,
+                                             None, None, None, ws.data_ptr(), n, H._stream()), "sage_qk_int8_sv_f16_attn_ws")
+    torch.cuda.synchronize()
+    assert not torch.isnan(ws).all()
+    assert torch.equal(o, want)
