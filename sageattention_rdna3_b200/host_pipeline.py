@@ -5,8 +5,8 @@ the copies about 10.  ``sageattn_host`` cuts q, k, v into chunks of whole (batch
 each an independent attention problem - and runs them through three CUDA streams: chunk i+1 is
 copied in while chunk i is computed and chunk i-1 is copied back, so the two PCIe directions and
 the GPU overlap.  The results are those of one ``sageattn`` call on device tensors (bit for bit
-when both take the same launch schedule).  16 chunks measured best for that shape (8.1 ms against
-8.4 with 8 and 9.1 with 32: finer chunks shorten the fill and drain of the pipeline until the host
+when both take the same launch schedule).  16 chunks measured best for that shape (8.22 ms against
+8.31 with 8 and 8.45 with 32: finer chunks shorten the fill and drain of the pipeline until the host
 side of the per-chunk calls shows).
 """
 from __future__ import annotations
@@ -65,13 +65,23 @@ def sageattn_host(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: Option
         s.wait_event(start)
     done_events = []
     outputs = []
-    for q_idx, kv_idx in slices:
+
+    def copy_in(q_idx, kv_idx):
         with torch.cuda.stream(s_in):
             qd_all[q_idx].copy_(q[q_idx], non_blocking=True)
             kd_all[kv_idx].copy_(k[kv_idx], non_blocking=True)
             vd_all[kv_idx].copy_(v[kv_idx], non_blocking=True)
             copied = torch.cuda.Event()
             copied.record(s_in)
+        return copied
+
+    # A chunk is copied back from the moment the next one has come in.  A copy-back that starts at some point within a
+    # copy-in slows both, by an amount that depends on where: delaying it by 0-100 us, a call with B=2 H=32 S=8192 took
+    # 8.06 to 8.78 ms, and faster launches alone had moved it from 8.17 to 8.48.  From the boundary on it takes
+    # 8.11-8.20 over the same delays; B=4 H=32 Hkv=8 S=4096 5.05 -> 4.45, B=2 H=16 S=4096 2.47 -> 2.30.
+    copied = copy_in(*slices[0]) if slices else None
+    for i, (q_idx, kv_idx) in enumerate(slices):
+        next_copied = copy_in(*slices[i + 1]) if i + 1 < len(slices) else None
         with torch.cuda.stream(s_run):
             s_run.wait_event(copied)
             od = sageattn(qd_all[q_idx].unsqueeze(0), kd_all[kv_idx].unsqueeze(0), vd_all[kv_idx].unsqueeze(0),
@@ -81,12 +91,15 @@ def sageattn_host(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: Option
             computed.record(s_run)
         with torch.cuda.stream(s_out):
             s_out.wait_event(computed)
+            if next_copied is not None:
+                s_out.wait_event(next_copied)
             od.record_stream(s_out)
             out[q_idx].copy_(od.squeeze(0), non_blocking=True)
             finished = torch.cuda.Event()
             finished.record(s_out)
             done_events.append(finished)
         outputs.append(od)
+        copied = next_copied
     for e in done_events:
         cur.wait_event(e)
     for t in (qd_all, kd_all, vd_all):
