@@ -1,11 +1,26 @@
 """Folding of the query heads of a GQA group into one row axis (csrc/internal.h) and the log-sum-exp
 correction for smooth_k (csrc/merge_kernels.cuh)."""
 import ctypes
+import subprocess
 
 import pytest
 import torch
 
 import helpers as H
+
+
+def _fold_rule(tmp_path):
+    """sage_gqa_fold(Hq, Hkv, Sq, o_stride_h, o_stride_s, is_causal), compiled for the host."""
+    from sageattention_rdna3_b200.build import CSRC
+    src = tmp_path / "fold.cpp"
+    src.write_text(f'#include "{CSRC}/internal.h"\n'
+                   'extern "C" int fold(long hq, long hkv, long sq, long sh, long ss, int c) '
+                   '{ return sage_gqa_fold(hq, hkv, sq, sh, ss, c); }\n')
+    lib = tmp_path / "fold.so"
+    subprocess.run(["g++", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
+    fold = ctypes.CDLL(str(lib)).fold
+    fold.argtypes = [ctypes.c_long] * 5 + [ctypes.c_int]
+    return fold
 
 
 @pytest.mark.gpu
@@ -15,10 +30,10 @@ import helpers as H
     (1, 3, 2, 64, 1000, 64, torch.float16),       # two heads fill a tile exactly
     (1, 2, 4, 31, 257, 128, torch.float16),       # heads end inside a 32-row scale group
     (2, 1, 8, 33, 129, 64, torch.bfloat16),       # two scale groups per head, the second of one row
-    (1, 2, 3, 127, 640, 128, torch.float16),      # a head is one row short of a tile
+    (1, 2, 3, 85, 640, 128, torch.float16),       # the folded rows are one short of two tiles
     (1, 2, 2, 160, 513, 64, torch.float16),       # more than a tile per head: 3 instead of 4 tiles
 ])
-def test_folded_heads_match_the_unfolded_launch(B, Hkv, rep, Sq, Skv, D, dtype, schedule):
+def test_folded_heads_match_the_unfolded_launch(tmp_path, B, Hkv, rep, Sq, Skv, D, dtype, schedule):
     """HND outputs are folded, NHD outputs (rows of a head not adjacent to the next head's) are not.  The
     same int8 values and scales: what differs is the rounding of P (fp16) where a warp holds other
     rows, and the order of the merge; the outputs are rounded to 16 bits once more."""
@@ -27,7 +42,10 @@ def test_folded_heads_match_the_unfolded_launch(B, Hkv, rep, Sq, Skv, D, dtype, 
     q = torch.randn(B, Hkv * rep, Sq, D, generator=g).to(dtype).cuda()
     k = (torch.randn(B, Hkv, Skv, D, generator=g) + 1.0).to(dtype).cuda()
     v = torch.randn(B, Hkv, Skv, D, generator=g).to(dtype).cuda()
-    nhd = [t.transpose(1, 2).contiguous() for t in (q, k, v)]
+    nhd = [t.transpose(1, 2).clone(memory_format=torch.contiguous_format) for t in (q, k, v)]
+    fold = _fold_rule(tmp_path)                   # the two launches that are compared are not the same one
+    assert fold(Hkv * rep, Hkv, Sq, q.stride(1), q.stride(2), 0) == rep
+    assert fold(Hkv * rep, Hkv, Sq, nhd[0].stride(2), nhd[0].stride(1), 0) == 1
     try:
         H.set_streamk(schedule)
         o, lse = sageattn_quantized_kv(q, quantize_kv(k, v, "HND", smooth_k=True), return_lse=True)
@@ -64,16 +82,7 @@ def test_lse_correction_against_64_bits(B, Hkv, rep, Sq, D, dtype, layout):
 
 def test_fold_rule_on_the_host(tmp_path):
     """The rule itself, compiled for the host: folded only where tiles are saved and the output allows it."""
-    import subprocess
-    from sageattention_rdna3_b200.build import CSRC
-    src = tmp_path / "fold.cpp"
-    src.write_text(f'#include "{CSRC}/internal.h"\n'
-                   'extern "C" int fold(long hq, long hkv, long sq, long sh, long ss, int c) '
-                   '{ return sage_gqa_fold(hq, hkv, sq, sh, ss, c); }\n')
-    lib = tmp_path / "fold.so"
-    subprocess.run(["g++", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
-    fold = ctypes.CDLL(str(lib)).fold
-    fold.argtypes = [ctypes.c_long] * 5 + [ctypes.c_int]
+    fold = _fold_rule(tmp_path)
     for sq in list(range(1, 300)) + [4096, 5000]:
         for hkv, rep in ((1, 1), (2, 2), (8, 4), (3, 8)):
             hq = hkv * rep

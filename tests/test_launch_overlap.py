@@ -23,10 +23,67 @@ def test_back_to_back_calls_on_buffers_that_change(D, S, smooth, dtype):
         for dst, src in zip((q, k, v), inputs[i % 4]):
             dst.copy_(src)
         got.append(sageattn(q, k, v, smooth_k=smooth))
+    torch.cuda.synchronize()
+    inner = sageattn(q, k, v, smooth_k=smooth)
+    torch.cuda.synchronize()                     # the value of the chain, with nothing overlapped
+    chain = sageattn(inner, k, v, smooth_k=smooth)
+    torch.cuda.synchronize()
     chained = [sageattn(sageattn(q, k, v, smooth_k=smooth), k, v, smooth_k=smooth) for _ in range(8)]
     torch.cuda.synchronize()
     assert all(torch.equal(o, want[i % 4]) for i, o in enumerate(got))
-    assert all(torch.equal(o, chained[0]) for o in chained)
+    assert all(torch.equal(o, chain) for o in chained)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", ["HND", "NHD"])
+@pytest.mark.parametrize("schedule", [0, 1])
+def test_cached_keys_back_to_back(layout, schedule):
+    """Four dependent kernels per call (Q, attention, merge, log-sum-exp), folded (HND) and not; the queries are
+    overwritten between calls, and the output of one call is the query of the next."""
+    import helpers
+    from sageattention_rdna3_b200 import quantize_kv, sageattn_quantized_kv
+    torch.manual_seed(1)
+    shape = lambda h, s: (2, h, s, 128) if layout == "HND" else (2, s, h, 128)
+    queries = [torch.randn(shape(8, 48), device="cuda").bfloat16() for _ in range(4)]
+    kv = quantize_kv(torch.randn(shape(2, 900), device="cuda").bfloat16() + 1, torch.randn(shape(2, 900), device="cuda").bfloat16(),
+                     layout, smooth_k=True)
+    try:
+        helpers.set_streamk(schedule)
+        want = []
+        for x in queries + [None]:
+            want.append(sageattn_quantized_kv(want[-1][0] if x is None else x, kv, return_lse=True))
+            torch.cuda.synchronize()
+        q, got = torch.empty_like(queries[0]), []
+        for i in range(32):
+            q.copy_(queries[i % 4])
+            got.append(sageattn_quantized_kv(q, kv, return_lse=True))
+            if i % 4 == 3:
+                got.append(sageattn_quantized_kv(got[-1][0], kv, return_lse=True))
+        torch.cuda.synchronize()
+    finally:
+        helpers.set_streamk(-1)
+    for i, (o, lse) in enumerate(got):
+        assert torch.equal(o, want[i % 5][0]) and torch.equal(lse, want[i % 5][1]), i
+
+
+@pytest.mark.gpu
+def test_two_streams_at_once():
+    """Calls on two streams whose kernels run beside each other: each gets its own results."""
+    from sageattention_rdna3_b200 import sageattn
+    torch.manual_seed(2)
+    work = [([torch.randn(1, 4, s, d, device="cuda").to(t) for _ in range(3)], kw, torch.cuda.Stream())
+            for s, d, t, kw in ((2304, 128, torch.bfloat16, dict(smooth_k=True)),
+                                (1500, 64, torch.float16, dict(is_causal=True, kernel="int8")))]
+    want = [sageattn(*x, **kw) for x, kw, _ in work]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(20):
+        for i, (x, kw, stream) in enumerate(work):
+            with torch.cuda.stream(stream):
+                got[i].append(sageattn(*x, **kw))
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert all(torch.equal(o, want[i]) for o in got[i])
 
 
 def test_nothing_shared_is_taken_before_the_kernel_ahead_has_ended():
