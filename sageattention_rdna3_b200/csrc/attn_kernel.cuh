@@ -347,8 +347,8 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   // preparation): with the allocation before the wait 18 of 110 SMs got two CTAs and 38 none, after it
   // every CTA has an SM to itself, as on an idle GPU.  4 heads of 4096 tokens, D=128: 62.1 -> 48.9 us per
   // call; 6 heads of 3072, un-quantised, D=64: 44.4 -> 33.0.  Causal launches of some 400-1000 items had
-  // gained from the uneven placement, which is given up: 16 heads of 4096 tokens 82.8 -> 90.1 us (97 with
-  // ordinary launches).
+  // gained from the uneven placement, which is given up: 16 heads of 4096 tokens 82.8 -> 90.1 us (95 with
+  // ordinary launches); a persistent launch, whose CTAs all start at once, pays about 0.5 us for the allocation.
   if (warp == 5) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();

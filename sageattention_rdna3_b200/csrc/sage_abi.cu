@@ -121,10 +121,12 @@ int encode_strided_16bit(CUtensorMap* map, CUtensorMapDataType dt, const void* b
 }
 
 // Launch with programmatic serialisation: the set-up of the kernel and its launch latency run under the end
-// of the kernel ahead of it in the stream (every kernel launched here begins with
-// grid_dependency_wait()).  A call is one to four kernels, most of them short.  Calls back to back, before
-// and after: 20 heads of 1024 tokens, D=64 19.4 -> 17.3 us, 10 heads of 4096 tokens 85.4 -> 81.3, 32 heads
-// of 4096 tokens causal, D=128 161 -> 154, B=2 H=32 S=8192 causal 944 -> 937.
+// of the kernel ahead of it in the stream.  Every kernel launched through here calls grid_dependency_wait() before
+// it touches global memory or takes TMEM (sage_fold_partial_kernel is an ordinary launch).  A call is one to
+// five kernels (K mean, preparation, attention, merge, log-sum-exp), most of them short, and conversions around
+// them for fp32 tensors.  Calls back to back, before and after: 20 heads of 1024 tokens, D=64 19.4 -> 17.2 us,
+// 10 heads of 4096 tokens 85.4 -> 82, 32 heads of 4096 tokens causal, D=128 159 -> 154; B=2 H=32 S=8192 causal is
+// level.
 template <typename... Params, typename... Args>
 int launch(void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
   cudaLaunchAttribute attr;
@@ -281,6 +283,8 @@ int plan_streamk(StreamKPlan* plan, int B, int Hq, int Sq, int Skv, int D, int i
                            static_cast<double>(std::min<long long>(items, 2 * grid)) * sage::kBlockM * D * 2) / 1e6;
   const double merge_steps = (5.0 + merge_mb / 4.0) / 1.95;
   // (1.04: the persistent CTAs of an SM run in lock-step, without the de-phasing yield of the plain launch)
+  // The constants were measured at head_dim 128 on the kernel before its tensor instructions moved behind
+  // elect.sync and its launches overlapped; they have not been fitted again, and head_dim 64 takes them as well.
   const double persistent = 1.04 * static_cast<double>(total) / grid + 5.0 + merge_steps;
   bool use = persistent < 0.95 * plain;
   if (forced == 1) use = true;
