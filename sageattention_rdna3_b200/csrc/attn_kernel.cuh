@@ -353,10 +353,6 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
-  // Only the persistent launch lets the next kernel (its merge) start early: blocks of a following
-  // preparation that wait beside the tail of a plain launch cost more than they gain (B=2 H=32 S=8192
-  // causal: 983 us per call with it, 937 without).
-  if (STREAMK) grid_launch_dependents();
   if (threadIdx.x == 0) {
     // A status word that is already set means an earlier CTA of this launch (or an earlier launch
     // the caller has not looked at yet) gave up: this CTA leaves through the abort path at once, so a
@@ -378,6 +374,11 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // Only the persistent launch lets the next kernel (its merge) start early: blocks of a following
+  // preparation that wait beside the tail of a plain launch cost more than they gain (B=2 H=32 S=8192
+  // causal: 983 us per call with it, 937 without).  Not before this CTA has its TMEM: the next kernel may
+  // take some as soon as it runs.
+  if (STREAMK) grid_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;
   const bool dead_on_arrival = *abort_flag != 0;
 

@@ -99,6 +99,9 @@ def test_nothing_shared_is_taken_before_the_kernel_ahead_has_ended():
     for word in ("tmem_alloc", "load_q(", "load_k(", "tma_load", "p.status", "p.q_scale", "__ldg", "atomic"):
         assert word not in before, word
     assert body.index("tmem_alloc(") > body.index("grid_dependency_wait();", setup)
+    # and the successor is not let in before the block has its own TMEM (the barrier behind the allocation)
+    alloc = body.index("tmem_alloc(")
+    assert body.index("grid_launch_dependents();") > body.index("__syncthreads();", alloc)
 
 
 @pytest.mark.gpu
