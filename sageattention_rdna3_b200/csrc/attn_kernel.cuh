@@ -74,6 +74,8 @@ struct AttnParams {
   int q_rows;                   // ... row r of it is row r % q_rows of head r / q_rows
   int n_q_tiles;
   int head_group;               // (batch, head) pairs scheduled together (a multiple of Hq/Hkv)
+  int tail_first, tail_size;    // causal plain launch: first pair and number of pairs of the last group, which has its own
+  int tail_block;               // ... size (sage_tail_group_first), and its first CTA
   int out_bf16;
   int qk_bf16;                  // un-quantised variant only: Q and K are bf16 (else fp16)
   float score_scale;            // un-quantised variant only: sm_scale * log2(e)
@@ -165,7 +167,7 @@ struct Segment {
 // STREAMK = false: one CTA = one whole item.  (batch, head) pairs are taken `head_group` at a time;
 // within a group the heaviest (last) query tiles go first and neighbouring CTAs are neighbouring
 // heads.  The CTAs resident at any moment then read the K/V of a few heads only (they stay in L2),
-// and the query heads of one KV head (GQA) run together.
+// and the query heads of one KV head (GQA) run together.  The last group of a causal launch is larger.
 // STREAMK = true: the KV-tile steps of all items, in (batch, head, query tile) order, form one line
 // of sk_total_tiles steps; CTA c owns steps [c*T/G, (c+1)*T/G) and walks through the items they
 // belong to: the tail of one item, whole items, the head of another.  All CTAs get the same amount
@@ -199,12 +201,16 @@ struct SegIter {
     if constexpr (!STREAMK) {
       if (!first) return false;
       first = false;
-      const int n_bh = p.B * p.Hq;
-      const int per_group = p.n_q_tiles * p.head_group;
-      const int group = blockIdx.x / per_group;
-      const int g_first = group * p.head_group;
-      const int g_size = min(p.head_group, n_bh - g_first);
-      const int within = blockIdx.x - group * per_group;
+      int g_first = p.tail_first, g_size = p.tail_size, within = blockIdx.x;
+      if (!CAUSAL || within < p.tail_block) {
+        const int per_group = p.n_q_tiles * p.head_group;
+        const int group = within / per_group;
+        g_first = group * p.head_group;
+        g_size = CAUSAL ? p.head_group : min(p.head_group, p.B * p.Hq - g_first);
+        within -= group * per_group;
+      } else {
+        within -= p.tail_block;
+      }
       const int qt = p.light_first ? within / g_size : p.n_q_tiles - 1 - within / g_size;
       fill(s, g_first + within % g_size, qt);
       const int kv_limit = CAUSAL ? min(s.q_base + kBlockM, p.Skv) : p.Skv;   // csrc/attn_gfx11.cu:502

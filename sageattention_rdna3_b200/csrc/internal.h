@@ -19,6 +19,23 @@ static inline int sage_gqa_fold(int64_t Hq, int64_t Hkv, int64_t Sq, int64_t o_s
   return (rows + 127) / 128 < rep * ((Sq + 127) / 128) ? (int)rep : 1;
 }
 
+// Order of the items (query tile, head) of a plain causal launch.  Heads go `head_group` at a time, the heaviest
+// (last) query tiles of a group first.  That balances the SMs as long as a group is followed by another one:
+// the next heavy items fill the gaps.  The last group has nothing behind it, so a small one - in particular
+// what is left over after whole groups - starts its heaviest items when the other SMs run dry.  The last group
+// therefore takes in whole groups before it until it has 1.5 items per CTA slot (two slots per SM), while the
+// keys and values of its heads (`kv_bytes` per head) stay in half of the L2.  Attention launch alone, us, groups of 8
+// throughout / with the larger last group: D=128 20 heads of 4096 tokens 101 / 83, 10 of 7000 164 / 126, 12 of 8192
+// 212 / 190, 64 of 3000 164 / 157, 64 of 2000 (un-quantised) 104 / 94; D=64 32 of 2048 (un-quantised) 44 / 36; where
+// the last group is large already (64 heads of 8192) 939 / 941.  One item per slot instead of 1.5: 24 heads of 2304 44
+// instead of 42.
+// Returns the first head of the last group, a multiple of head_group.
+static inline int sage_tail_group_first(int n_heads, int head_group, int n_q_tiles, double kv_bytes, int sms) {
+  int tail = n_heads % head_group;
+  while (tail < n_heads && (long long)tail * n_q_tiles < 3LL * sms && (tail + head_group) * kv_bytes <= 64e6) tail += head_group;
+  return n_heads - tail;
+}
+
 extern "C" {
 // lse[b,h,s] += sm_scale * q[b,h,s,:] . k_mean[b, h / (Hq/Hkv), :], in fp32: refers the log-sum-exp of a
 // launch on centred keys (smooth_k) to the original ones.  lse: contiguous [B,Hq,Sq]; k_mean:

@@ -196,6 +196,27 @@ void fill_attn_params(sage::AttnParams* pp, void* o, int64_t o_stride_b, int64_t
   p.test_drop_v_load = (g_test_drop_v_load.load(std::memory_order_relaxed) != 0 && limit < sage::kWaitLimitCycles) ? 1 : 0;
 }
 
+int sm_count(int* out);
+
+// Order of the items of a plain causal launch.  Scattering launches keep groups of one size: their order is
+// chosen for the links (light_first).
+int set_item_order(sage::AttnParams* pp, int D, int kv_bytes_per_element) {
+  sage::AttnParams& p = *pp;
+  const int n_bh = p.B * p.Hq;
+  p.tail_first = n_bh / p.head_group * p.head_group;
+  if (p.n_peers == 0) {
+    int sms = 0;
+    const int rc = sm_count(&sms);
+    if (rc) return rc;
+    const double kv_bytes = static_cast<double>(p.Skv) * D * kv_bytes_per_element * p.Hkv / p.Hq;
+    p.tail_first = sage_tail_group_first(n_bh, p.head_group, p.n_q_tiles, kv_bytes, sms);
+  }
+  p.tail_size = n_bh - p.tail_first;
+  // (a grid that does not fit an int is refused before the launch)
+  p.tail_block = static_cast<int>(std::min<long long>(0x7fffffffLL, static_cast<long long>(p.tail_first) * p.n_q_tiles));
+  return SAGE_OK;
+}
+
 int sm_count(int* out) {
   static std::atomic<int> cached[64];
   int dev = 0;
@@ -759,6 +780,11 @@ int attn_int8_impl(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t*
     }
   }
 
+  if (is_causal) {
+    const int rc = set_item_order(&p, D, 3);              // int8 K, fp16 V
+    if (rc) return rc;
+  }
+
   // With no keys every row has l == 0 and the output is 0 (csrc/attn_gfx11.cu:771).  The kernel
   // handles that without touching K or V, but a tensor map cannot have a zero extent: describe one
   // dummy row instead (it is never loaded).
@@ -931,8 +957,13 @@ int direct_attn_impl(const sage_strided_t* q, const sage_strided_t* k, const sag
   fill_attn_params(&p, o, o_stride_b, o_stride_h, o_stride_s, dtype, B, Hq, Hkv, Sq, Skv, lse, status);
   p.qk_bf16 = (dtype == SAGE_DTYPE_BF16);
   p.score_scale = sm_scale * 1.4426950408889634f;       // csrc/attn_gfx11.cu:34, as for the quantised path
-  p.n_peers = n_peers;                                  // (short sequences: the order of the items is left alone)
+  p.n_peers = n_peers;                                  // (short sequences: never the lightest items first)
   for (int i = 0; i < n_peers; ++i) p.peer_o[i] = peer_o[i];
+  int rc = SAGE_OK;
+  if (is_causal) {
+    rc = set_item_order(&p, D, 4);
+    if (rc) return rc;
+  }
 
   // No keys: nothing is loaded (see sage_qk_int8_sv_f16_attn_lse); the maps describe one dummy row.
   const int skv_map = Skv > 0 ? Skv : 1;
@@ -943,7 +974,7 @@ int direct_attn_impl(const sage_strided_t* q, const sage_strided_t* k, const sag
   const CUtensorMapDataType qk_dt = p.qk_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
 
   CUtensorMap tq, tk, tv, to;
-  int rc = encode_strided_16bit(&tq, qk_dt, q->ptr, D, Sq, Hq, B, q->stride_s, q->stride_h, q->stride_b, sage::kBlockM, "q");
+  rc = encode_strided_16bit(&tq, qk_dt, q->ptr, D, Sq, Hq, B, q->stride_s, q->stride_h, q->stride_b, sage::kBlockM, "q");
   if (rc) return rc;
   rc = encode_strided_16bit(&tk, qk_dt, k_base, D, skv_map, Hkv, B, kk.stride_s, kk.stride_h, kk.stride_b, sage::kBlockN, "k");
   if (rc) return rc;
