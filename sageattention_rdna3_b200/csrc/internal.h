@@ -36,6 +36,22 @@ static inline int sage_tail_group_first(int n_heads, int head_group, int n_q_til
   return n_heads - tail;
 }
 
+// Persistent or plain launch under a causal mask.  The plain launch takes as long as its heaviest item, a CTA by
+// itself for most of the time (5 us + 1.15 us per KV tile), or as all items together on all slots (two CTAs per SM,
+// 6 us + 2 us per tile and slot), whichever is more; its items come heaviest first, so the two do not add up.  The
+// persistent launch cuts the steps into equal spans, but a span in the light end of a head is many items of one to
+// a few tiles, each with its own start and end, and that span is the last to finish.  So it pays only where the heaviest item alone
+// is far above the mean: few heads, long ones.  Plain / persistent, us, attention launch with its merge (n heads of
+// t tiles): D=64 1 of 64 79 / 36, 2 of 48 61 / 37, 4 of 40 58 / 52, 5 of 24 38 / 40, 14 of 24 38 / 58; D=128 1 of 64 80 / 45,
+// 2 of 40 53 / 40, 3 of 32 47 / 43, 4 of 40 55 / 60, 10 of 24 37 / 62; un-quantised within a few per cent of that.
+// heads: (batch, query head) pairs; heaviest: KV tiles of the heaviest item; mean_steps: KV tiles per CTA of the
+// persistent launch.
+static inline int sage_causal_streamk(int64_t heads, int64_t heaviest, double mean_steps, int D) {
+  if (heads > (D == 64 ? 4 : 3) || heaviest < 2.2 * mean_steps) return 0;
+  const int fewest = D == 64 ? (heads <= 2 ? 8 : 20) : (heads == 1 ? 8 : heads == 2 ? 24 : 32);
+  return heaviest >= fewest;
+}
+
 extern "C" {
 // lse[b,h,s] += sm_scale * q[b,h,s,:] . k_mean[b, h / (Hq/Hkv), :], in fp32: refers the log-sum-exp of a
 // launch on centred keys (smooth_k) to the original ones.  lse: contiguous [B,Hq,Sq]; k_mean:

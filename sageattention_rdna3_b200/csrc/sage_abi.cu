@@ -257,7 +257,7 @@ int streamk_override() {
 // The persistent launch cuts the T = sum of KV-tile steps into 2 * SMs equal spans instead; a span
 // that covers part of an item leaves a partial result in the workspace and a merge kernel combines
 // them.  It costs about three KV-tile steps per CTA (a second pipeline fill and drain, the merge), so
-// it is used when the estimate says it saves at least 8 %.
+// it is used only where the rules in plan_streamk say that it saves more.
 struct StreamKPlan {
   bool use = false;
   int grid = 0;
@@ -286,28 +286,28 @@ int plan_streamk(StreamKPlan* plan, int B, int Hq, int Sq, int Skv, int D, int i
   const long long total = per_head * B * Hq;
   if (per_head > 0x7fffffffLL || items > 0x7fffffffLL) return SAGE_OK;
   const long long grid = total < slots ? total : slots;
-  // Makespans in KV-tile steps of a CTA that shares its SM with another one.  Plain launch: full
-  // waves of `slots` items, then a tail wave that runs about 1.4x faster per CTA if it leaves every
-  // CTA alone on its SM; under a causal mask the heavy-first order packs items almost evenly.  About
-  // 3 steps of fixed cost per wave (set-up, pipeline fill and drain, epilogue).  Persistent launch:
-  // 1.04 T / G steps, the same fixed cost once, two more pipeline restarts at item boundaries, and the
-  // merge (about 5 us plus its traffic at 4 TB/s; one step is about 1.95 us).
-  double plain;
+  bool use;
   if (is_causal) {
-    plain = std::max<double>(static_cast<double>(std::min(nq, nkv)), 1.03 * total / slots) + 3.0;
+    use = sage_causal_streamk(static_cast<long long>(B) * Hq, std::min(nq, nkv), static_cast<double>(total) / grid, D) != 0;
   } else {
+    // Makespans in KV-tile steps of a CTA that shares its SM with another one.  Plain launch: full
+    // waves of `slots` items, then a tail wave that runs about 1.4x faster per CTA if it leaves every
+    // CTA alone on its SM.  About 3 steps of fixed cost per wave (set-up, pipeline fill and drain, epilogue).
+    // Persistent launch: 1.04 T / G steps, the same fixed cost once, two more pipeline restarts at item
+    // boundaries, and the merge (about 5 us plus its traffic at 4 TB/s; one step is about 1.95 us).
+    // (1.04: the persistent CTAs of an SM run in lock-step, without the de-phasing yield of the plain launch)
+    // The constants were measured at head_dim 128 on an earlier kernel.  Checked on the present one, both launches
+    // timed for 892 combinations of 2-800 items, 2-128 tiles, both kernels and head sizes: the choice is 0.3 %
+    // behind the better of the two on average.
     const long long full = items / slots, tail = items % slots;
-    plain = static_cast<double>(full) * (nkv + 3.0);
+    double plain = static_cast<double>(full) * (nkv + 3.0);
     if (tail > 0) plain += (tail <= sms ? 0.72 : 1.0) * nkv + 3.0;
+    const double merge_mb = (static_cast<double>(grid) * 2 * sage::kBlockM * D * 4 +
+                             static_cast<double>(std::min<long long>(items, 2 * grid)) * sage::kBlockM * D * 2) / 1e6;
+    const double merge_steps = (5.0 + merge_mb / 4.0) / 1.95;
+    const double persistent = 1.04 * static_cast<double>(total) / grid + 5.0 + merge_steps;
+    use = persistent < 0.95 * plain;
   }
-  const double merge_mb = (static_cast<double>(grid) * 2 * sage::kBlockM * D * 4 +
-                           static_cast<double>(std::min<long long>(items, 2 * grid)) * sage::kBlockM * D * 2) / 1e6;
-  const double merge_steps = (5.0 + merge_mb / 4.0) / 1.95;
-  // (1.04: the persistent CTAs of an SM run in lock-step, without the de-phasing yield of the plain launch)
-  // The constants were measured at head_dim 128 on the kernel before its tensor instructions moved behind
-  // elect.sync and its launches overlapped; they have not been fitted again, and head_dim 64 takes them as well.
-  const double persistent = 1.04 * static_cast<double>(total) / grid + 5.0 + merge_steps;
-  bool use = persistent < 0.95 * plain;
   if (forced == 1) use = true;
   if (!use) return SAGE_OK;
   plan->use = true;

@@ -1,4 +1,5 @@
-"""Order of the items of a plain causal launch: the last group of heads has its own size (csrc/internal.h)."""
+"""Schedule of causal launches (csrc/internal.h): the last group of heads of a plain launch has its own size, and which
+launches are persistent."""
 import ctypes
 import subprocess
 
@@ -8,22 +9,24 @@ import torch
 import helpers as H
 
 
-def _tail_rule(tmp_path):
+def _rules(tmp_path):
     from sageattention_rdna3_b200.build import CSRC
-    src = tmp_path / "tail.cpp"
+    src = tmp_path / "rules.cpp"
     src.write_text(f'#include "{CSRC}/internal.h"\n'
-                   'extern "C" int tail(int n, int g, int nq, double b, int sms) { return sage_tail_group_first(n, g, nq, b, sms); }\n')
-    lib = tmp_path / "tail.so"
+                   'extern "C" int tail(int n, int g, int nq, double b, int sms) { return sage_tail_group_first(n, g, nq, b, sms); }\n'
+                   'extern "C" int streamk(long n, long t, double m, int d) { return sage_causal_streamk(n, t, m, d); }\n')
+    lib = tmp_path / "rules.so"
     subprocess.run(["g++", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
-    tail = ctypes.CDLL(str(lib)).tail
-    tail.argtypes = [ctypes.c_int] * 3 + [ctypes.c_double, ctypes.c_int]
-    return tail
+    rules = ctypes.CDLL(str(lib))
+    rules.tail.argtypes = [ctypes.c_int] * 3 + [ctypes.c_double, ctypes.c_int]
+    rules.streamk.argtypes = [ctypes.c_long, ctypes.c_long, ctypes.c_double, ctypes.c_int]
+    return rules
 
 
 def test_every_item_has_one_block(tmp_path):
     """The kernel's map from block to (head, query tile), for whole GQA groups, odd numbers of heads, one tile, and
     heads too large to share the L2."""
-    tail = _tail_rule(tmp_path)
+    tail = _rules(tmp_path).tail
     for n_heads in (1, 3, 7, 8, 9, 20, 24, 63, 128):
         for group in (8, 9, 12):
             for nq in (1, 2, 18, 64):
@@ -39,6 +42,16 @@ def test_every_item_has_one_block(tmp_path):
                             g_first, size, within = first, n_heads - first, block - first * nq
                         items.add((g_first + within % size, nq - 1 - within // size))
                     assert items == {(h, t) for h in range(n_heads) for t in range(nq)}
+
+
+@pytest.mark.parametrize("heads,tiles,D,persistent", [
+    (1, 7, 64, 0), (1, 8, 64, 1), (4, 19, 64, 0), (4, 20, 64, 1), (5, 40, 64, 0), (4, 96, 64, 0),
+    (1, 7, 128, 0), (1, 8, 128, 1), (2, 23, 128, 0), (2, 24, 128, 1), (3, 31, 128, 0), (3, 32, 128, 1), (4, 40, 128, 0),
+    (10, 24, 128, 0), (64, 64, 128, 0),
+])
+def test_few_long_causal_heads_are_cut_into_spans(tmp_path, heads, tiles, D, persistent):
+    steps = heads * tiles * (tiles + 1) // 2
+    assert _rules(tmp_path).streamk(heads, tiles, steps / min(steps, 296), D) == persistent
 
 
 @pytest.mark.gpu
