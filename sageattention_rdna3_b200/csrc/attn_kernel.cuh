@@ -582,12 +582,6 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       asm volatile("bar.sync 1, 128;" ::: "memory");      // the four softmax warps only
       yields = (*arrival & 1u) != 0u;
     }
-    // A step that moves the maximum waits for the P.V of the half before and scales O.  int8: behind the exp pass, under
-    // which that P.V completes (x20 outliers, attention launch: 16 heads of 4096 tokens, D=128 166 -> 157 us, 32 / 8 heads
-    // of 4 x 4096 causal 643 -> 628; without outliers level).  Un-quantised: ahead of it (61 us against 72 for 20
-    // heads of 2048 with outliers, D=64).  The causal kernel, larger by the masked tiles, keeps the loop over O rolled.
-    constexpr bool kRescaleFirst = QKF;
-    constexpr int kRescaleUnroll = (CAUSAL && !QKF) ? 1 : D / 32;
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
     const uint32_t t_o = tmem_base + lane_base + kColO;
     bool ok = true;
@@ -733,51 +727,77 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           }
       }
 
-      // O *= alpha.  O must be at rest: the P.V of the previous half has to be complete.
-      auto rescale_o = [&](float alpha) -> bool {
-        const int hp = h ^ 1;
-        const int tp = h ? t : t - 1;
-        SAGE_WAIT_OR(pv_done + hp, tp & 1, 9, return false);
-        tc_fence_after();
-#pragma unroll kRescaleUnroll
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t orr[32];
-          tmem_ld32(t_o + 32 * c, orr);
-          tc_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) orr[i] = __float_as_uint(__uint_as_float(orr[i]) * alpha);
-          tmem_st32(t_o + 32 * c, orr);
-        }
-        return true;
-      };
-      if (!done) {
-        // lazy rescale: move the running maximum only when it grew by more than 2^14
-        bool moved = false;
-        float alpha = 1.0f;
-        if (hh == 0) {
-          m_used = m_half;
-        } else {
-          // After a refused attempt the bar is lower: a row whose 64 values added up to more
-          // than 2^14 has a maximum above 2^8, and it must move or it would be refused again.
-          const bool need = m_half > m_used + (attempt ? kRefusedBarLog2 : kLazyRescaleLog2);
-          moved = __any_sync(0xffffffffu, need);
-          if (!attempt) distrust = moved ? min(distrust + 1, 4) : distrust - 1;
-          if (need) {
-            alpha = fast_exp2(m_used - m_half);                             // (:667)
+      // A step that is not done yet.  Lazy rescale: the running maximum moves only when it grew by more than 2^14; after
+      // a refused attempt the bar is lower: a row whose 64 values added up to more than 2^14 has a maximum above
+      // 2^8, and it must move or it would be refused again.  A warp in which a row moves scales O, which must be
+      // at rest for that: the P.V of the previous half has to be complete.
+      // Un-quantised: O first, then the exponentials.  int8: the exponentials first, under which that P.V completes
+      // (x20 outliers, attention launch: 16 heads of 4096 tokens, D=128 167 -> 157 us, 4 x 32 / 8 heads of 4096 causal
+      // 643 -> 626; without outliers level.  Un-quantised, 20 heads of 2048 with outliers, D=64, it would be 61 -> 72).
+      // The causal kernel, which is larger by the masked tiles, keeps the loop over O rolled.  (Written out twice: one
+      // copy with a switch compiled to a kernel 1 % slower without outliers.)
+      if constexpr (QKF) {
+        if (!done) {
+          if (hh == 0) {
             m_used = m_half;
+          } else {
+            const bool need = m_half > m_used + (attempt ? kRefusedBarLog2 : kLazyRescaleLog2);
+            const bool moved = __any_sync(0xffffffffu, need);
+            if (!attempt) distrust = moved ? min(distrust + 1, 4) : distrust - 1;
+            if (moved) {
+              const int hp = h ^ 1;
+              const int tp = h ? t : t - 1;
+              SAGE_WAIT_OR(pv_done + hp, tp & 1, 9, { ok = false; break; });
+              tc_fence_after();
+              const float alpha = need ? fast_exp2(m_used - m_half) : 1.0f;   // (:667)
+              if (need) m_used = m_half;
+              l *= alpha;
+#pragma unroll
+              for (int c = 0; c < D / 32; ++c) {
+                uint32_t orr[32];
+                tmem_ld32(t_o + 32 * c, orr);
+                tc_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; ++i) orr[i] = __float_as_uint(__uint_as_float(orr[i]) * alpha);
+                tmem_st32(t_o + 32 * c, orr);
+              }
+            }
+          }
+          // Two copies of the loop: only tiles on the diagonal or at the ragged end pay for masking.
+          if (masked) l += exp_pass(std::true_type{}, m_used);
+          else l += exp_pass(std::false_type{}, m_used);
+        }
+      } else {
+        if (!done) {
+          bool moved = false;
+          float alpha = 1.0f;
+          if (hh == 0) {
+            m_used = m_half;
+          } else {
+            const bool need = m_half > m_used + (attempt ? kRefusedBarLog2 : kLazyRescaleLog2);
+            moved = __any_sync(0xffffffffu, need);
+            if (!attempt) distrust = moved ? min(distrust + 1, 4) : distrust - 1;
+            alpha = need ? fast_exp2(m_used - m_half) : 1.0f;                 // (:667)
+            if (need) m_used = m_half;
             l *= alpha;
           }
-          if (kRescaleFirst && moved && !rescale_o(alpha)) {
-            ok = false;
-            break;
+          if (masked) l += exp_pass(std::true_type{}, m_used);
+          else l += exp_pass(std::false_type{}, m_used);
+          if (moved) {
+            const int hp = h ^ 1;
+            const int tp = h ? t : t - 1;
+            SAGE_WAIT_OR(pv_done + hp, tp & 1, 9, { ok = false; break; });
+            tc_fence_after();
+#pragma unroll(CAUSAL ? 1 : D / 32)
+            for (int c = 0; c < D / 32; ++c) {
+              uint32_t orr[32];
+              tmem_ld32(t_o + 32 * c, orr);
+              tc_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) orr[i] = __float_as_uint(__uint_as_float(orr[i]) * alpha);
+              tmem_st32(t_o + 32 * c, orr);
+            }
           }
-        }
-        // Two copies of the loop: only tiles on the diagonal or at the ragged end pay for masking.
-        if (masked) l += exp_pass(std::true_type{}, m_used);
-        else l += exp_pass(std::false_type{}, m_used);
-        if (!kRescaleFirst && moved && !rescale_o(alpha)) {
-          ok = false;
-          break;
         }
       }
       tmem_st32(tmem_base + lane_base + kColP + h * kHalfN, pk);
