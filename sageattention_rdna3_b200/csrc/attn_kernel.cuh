@@ -963,24 +963,25 @@ struct MergeParams {
   int causal, out_bf16;
 };
 
-// ROWS: rows of an item per merge CTA.  32 (four 16-byte pieces per thread) when there are many items;
-// the loop over the parts is a chain of loads, so with few items - long ones, in many parts - the
-// fewest rows a CTA can take, for as many CTAs as possible: 64 items of 64 steps in 5-6 parts, D=128,
-// 68.3 -> 64.7 us per call.
+// ROWS: rows of an item per merge CTA, CHUNK: parts whose loads are in flight together.  A thread owns 16-byte pieces of
+// one to four rows and works out the weights of its rows itself, so there is one round trip to the L2 per CHUNK parts
+// and no exchange between threads.  Many items have few parts each (32 rows, two parts at a time); with few items -
+// long ones, in many parts - the CTAs take the fewest rows that fill their threads, for as many CTAs as possible.
+// Attention launch and merge, us, against a merge that fetched one part after the other, weights first: 64 items of 64
+// tiles (5-6 parts each), D=128 54.5 -> 50.8; 16 items of 32 tiles 26.3 -> 20.8; 2 causal heads of 4096 tokens 34.7 -> 30.5;
+// 320 items of 32, D=64 77.1 -> 76.1; 320 of 16, D=64 45.4 -> 44.4; 512 of 128 level.  Four parts at a time for many
+// items: 77.6 and 46.1.
 constexpr int kMergeRows = 32;
+constexpr int kMergeChunk = 2;
+constexpr int kMergeChunkFew = 8;
 __host__ __device__ constexpr int merge_rows_few(int D) { return 256 * 4 / D; }
 
-template <int D, int ROWS>
+template <int D, int ROWS, int CHUNK>
 __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams p) {
-  __shared__ float row_max[ROWS];
-  __shared__ float row_inv[ROWS];
-  grid_dependency_wait();
-  grid_launch_dependents();
   const int item = blockIdx.x / (kBlockM / ROWS);
   const int row0 = (blockIdx.x - item * (kBlockM / ROWS)) * ROWS;     // first row of this CTA within the item
   const int bh = item / p.n_q_tiles;
   const int qt = item - bh * p.n_q_tiles;
-  if (qt * kBlockM + row0 >= p.Sq) return;
   const int nkv = p.nkv_full;
   const int tiles = p.causal ? min(qt + 1, nkv) : nkv;
   long long before;                                      // steps of this head before query tile qt
@@ -992,63 +993,76 @@ __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams 
   const long long G = p.attn_grid, T = p.total_tiles;
   const int c_first = static_cast<int>(((start + 1) * G - 1) / T);     // CTA that owns step `start`
   const int c_last = static_cast<int>((end * G - 1) / T);              // ... step `end - 1`
-  if (c_first == c_last) return;
   const int n_parts = c_last - c_first + 1;
   const int first_slot = ((T * c_first) / G == start) ? 0 : 1;
-  // rows of part k start at this offset (in rows) of the partial buffers
-  auto part_row0 = [&](int k) -> long long {
-    return (static_cast<long long>(c_first + k) * 2 + (k == 0 ? first_slot : 0)) * kBlockM + row0;
-  };
+  grid_dependency_wait();                                // (all of the above is arithmetic on the arguments)
+  grid_launch_dependents();
+  if (n_parts == 1 || qt * kBlockM + row0 >= p.Sq) return;
 
-  const int tid = threadIdx.x;
-  if (tid < ROWS) {
-    float e_max = -INFINITY;
-    for (int k = 0; k < n_parts; ++k) e_max = fmaxf(e_max, p.part_lse[part_row0(k) + tid]);
-    float sum = 0.0f;
-    for (int k = 0; k < n_parts; ++k) {
-      const float e = p.part_lse[part_row0(k) + tid];
-      sum += (e == -INFINITY) ? 0.0f : exp2f(e - e_max);
-    }
-    row_max[tid] = e_max;
-    row_inv[tid] = (sum > 0.0f) ? 1.0f / sum : 0.0f;
-    const int row = qt * kBlockM + row0 + tid;
-    if (p.lse != nullptr && row < p.Sq) {
-      p.lse[static_cast<long long>(bh) * p.Sq + row] =
-          (sum > 0.0f) ? (e_max + log2f(sum)) * 0.6931471805599453f : -INFINITY;
-    }
-  }
-  __syncthreads();
-  const int b = bh / p.Hq, h = bh - b * p.Hq;
   constexpr int kVecPerRow = D / 4;
-  constexpr int kPerThread = ROWS * kVecPerRow / 256;   // float4 per thread: 1, 2 or 4
+  constexpr int kPerThread = ROWS * kVecPerRow / 256;    // float4 per thread: 1, 2 or 4
+  constexpr int kRowStep = 256 / kVecPerRow;
+  const int r0 = threadIdx.x / kVecPerRow, c4 = threadIdx.x % kVecPerRow;   // rows r0, r0 + kRowStep, ...
+  // the first part may be the last segment of its CTA (slot 1), the others are the first of theirs (slot 0)
+  const long long row_first = (static_cast<long long>(c_first) * 2 + first_slot) * kBlockM + row0 + r0;
+  const long long row_other = static_cast<long long>(c_first) * 2 * kBlockM + row0 + r0;
+  float e_max[kPerThread], sum[kPerThread];
   float4 acc[kPerThread];
 #pragma unroll
-  for (int u = 0; u < kPerThread; ++u) acc[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  for (int k = 0; k < n_parts; ++k) {
-    const long long pr = part_row0(k);
-    float4 x[kPerThread];
-    float w[kPerThread];
+  for (int u = 0; u < kPerThread; ++u) {
+    e_max[u] = -INFINITY;
+    sum[u] = 0.0f;
+    acc[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+#pragma unroll 1
+  for (int k0 = 0; k0 < n_parts; k0 += CHUNK) {
+    float e[CHUNK][kPerThread];
+    float4 x[CHUNK][kPerThread];
 #pragma unroll
-    for (int u = 0; u < kPerThread; ++u) {
-      const int idx = tid + u * 256;
-      const int r = idx / kVecPerRow, c4 = idx - r * kVecPerRow;
-      const float e = p.part_lse[pr + r];
-      w[u] = (e == -INFINITY) ? 0.0f : exp2f(e - row_max[r]);
-      x[u] = *reinterpret_cast<const float4*>(p.part_o + (pr + r) * D + 4 * c4);
+    for (int c = 0; c < CHUNK; ++c) {
+      const int k = k0 + c;
+      const long long pr = k == 0 ? row_first : row_other + static_cast<long long>(k) * 2 * kBlockM;
+#pragma unroll
+      for (int u = 0; u < kPerThread; ++u) {
+        e[c][u] = -INFINITY;
+        x[c][u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (k < n_parts) {
+          e[c][u] = p.part_lse[pr + u * kRowStep];
+          x[c][u] = *reinterpret_cast<const float4*>(p.part_o + (pr + u * kRowStep) * D + 4 * c4);
+        }
+      }
     }
 #pragma unroll
     for (int u = 0; u < kPerThread; ++u) {
-      if (w[u] == 0.0f) continue;                         // a part without visible keys may hold anything
-      acc[u].x += w[u] * x[u].x; acc[u].y += w[u] * x[u].y; acc[u].z += w[u] * x[u].z; acc[u].w += w[u] * x[u].w;
+      float top = e_max[u];
+#pragma unroll
+      for (int c = 0; c < CHUNK; ++c) top = fmaxf(top, e[c][u]);
+      if (top == -INFINITY) continue;                    // no visible keys so far
+      if (k0 > 0) {
+        const float back = exp2f(e_max[u] - top);
+        sum[u] *= back;
+        acc[u].x *= back; acc[u].y *= back; acc[u].z *= back; acc[u].w *= back;
+      }
+      e_max[u] = top;
+#pragma unroll
+      for (int c = 0; c < CHUNK; ++c) {
+        const float w = exp2f(e[c][u] - top);            // 0 for a part without visible keys
+        if (w == 0.0f) continue;                         // ... which may hold anything
+        sum[u] += w;
+        acc[u].x += w * x[c][u].x; acc[u].y += w * x[c][u].y; acc[u].z += w * x[c][u].z; acc[u].w += w * x[c][u].w;
+      }
     }
   }
+  const int b = bh / p.Hq, h = bh - b * p.Hq;
 #pragma unroll
   for (int u = 0; u < kPerThread; ++u) {
-    const int idx = tid + u * 256;
-    const int r = idx / kVecPerRow, c4 = idx - r * kVecPerRow;
-    const int row = qt * kBlockM + row0 + r;
+    const int row = qt * kBlockM + row0 + r0 + u * kRowStep;
     if (row >= p.Sq) continue;
-    const float inv = row_inv[r];
+    const float inv = (sum[u] > 0.0f) ? 1.0f / sum[u] : 0.0f;
+    if (p.lse != nullptr && c4 == 0) {
+      p.lse[static_cast<long long>(bh) * p.Sq + row] =
+          (sum[u] > 0.0f) ? (e_max[u] + log2f(sum[u])) * 0.6931471805599453f : -INFINITY;
+    }
     const long long off = b * p.o_stride_b + h * p.o_stride_h + static_cast<long long>(row) * p.o_stride_s + 4 * c4;
     uint2 out;
     if (p.out_bf16) {

@@ -376,9 +376,9 @@ int launch_attn_streamk(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   const long long items = static_cast<long long>(p.n_q_tiles) * p.B * p.Hq;
   constexpr int kFew = sage::merge_rows_few(D);
   if (items <= kFewMergeItems) {
-    return launch(sage::sage_attn_merge_kernel<D, kFew>, static_cast<unsigned>(items * (sage::kBlockM / kFew)), 256, 0, stream, m);
+    return launch(sage::sage_attn_merge_kernel<D, kFew, sage::kMergeChunkFew>, static_cast<unsigned>(items * (sage::kBlockM / kFew)), 256, 0, stream, m);
   }
-  return launch(sage::sage_attn_merge_kernel<D, sage::kMergeRows>,
+  return launch(sage::sage_attn_merge_kernel<D, sage::kMergeRows, sage::kMergeChunk>,
                 static_cast<unsigned>(items * (sage::kBlockM / sage::kMergeRows)), 256, 0, stream, m);
 }
 
