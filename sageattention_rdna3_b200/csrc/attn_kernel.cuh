@@ -81,6 +81,8 @@ struct AttnParams {
   float score_scale;            // un-quantised variant only: sm_scale * log2(e)
   int32_t* s_dump;              // optional [B,Hq,Sq,Skv] int32 copy of Q.K^T (debug / parity)
   float* lse;                   // optional [B,Hq,Sq]: natural-log sum of exp of the scaled scores
+  int lse_add;                  // 1: ... added to lse_add_scale times what `lse` holds
+  float lse_add_scale;
   int* status;                  // optional device word, stays 0 on success
   int* status_host;             // optional word in mapped pinned host memory that receives the same code
   long long wait_limit_cycles;  // bound of every barrier wait, in SM clocks
@@ -826,8 +828,9 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (p.lse != nullptr && row < p.Sq) {
           // scores are in base 2 (log2(e) is folded into the Q scale): ln sum exp = (m + log2 l) ln 2;
           // a row without keys gets -inf
-          p.lse[static_cast<long long>(bh) * p.Sq + row] =
-              (l > 0.0f) ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
+          const float lse = (l > 0.0f) ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
+          float* dst = p.lse + static_cast<long long>(bh) * p.Sq + row;
+          *dst = p.lse_add ? fmaf(p.lse_add_scale, *dst, lse) : lse;
         }
       } else {
         p.part_lse[(static_cast<long long>(blockIdx.x) * 2 + sg.slot) * kBlockM + threadIdx.x] =
@@ -956,6 +959,8 @@ struct MergeParams {
   void* o;
   long long o_stride_b, o_stride_h, o_stride_s;
   float* lse;                   // optional [B,Hq,Sq]
+  int lse_add;                  // as in AttnParams
+  float lse_add_scale;
   int Hq, Sq, n_q_tiles;
   int nkv_full, tiles_per_head;
   long long total_tiles;
@@ -1060,8 +1065,9 @@ __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams 
     if (row >= p.Sq) continue;
     const float inv = (sum[u] > 0.0f) ? 1.0f / sum[u] : 0.0f;
     if (p.lse != nullptr && c4 == 0) {
-      p.lse[static_cast<long long>(bh) * p.Sq + row] =
-          (sum[u] > 0.0f) ? (e_max[u] + log2f(sum[u])) * 0.6931471805599453f : -INFINITY;
+      const float lse = (sum[u] > 0.0f) ? (e_max[u] + log2f(sum[u])) * 0.6931471805599453f : -INFINITY;
+      float* dst = p.lse + static_cast<long long>(bh) * p.Sq + row;
+      *dst = p.lse_add ? fmaf(p.lse_add_scale, *dst, lse) : lse;
     }
     const long long off = b * p.o_stride_b + h * p.o_stride_h + static_cast<long long>(row) * p.o_stride_s + 4 * c4;
     uint2 out;

@@ -58,6 +58,16 @@ extern "C" {
 // contiguous [B,Hkv,D] in the dtype of q.
 int sage_lse_add_q_mean(const sage_strided_t* q, int dtype, const void* k_mean, float* lse, int B, int Hq, int Hkv, int Sq,
                         int D, float sm_scale, void* stream);
+// The same without a launch of its own: sage_quant_q_mean_dot quantises Q like sage_quant_qk_int8 and leaves
+// q[b,h,s,:] . k_mean[b, h / (Hq/Hkv), :] in lse, and sage_qk_int8_sv_f16_attn_lse_add, which is
+// sage_qk_int8_sv_f16_attn_ws otherwise, adds lse_add_scale times that to what it writes there.
+int sage_quant_q_mean_dot(const sage_strided_t* q, int dtype, const void* k_mean, int B, int Hq, int Hkv, int Sq, int D,
+                          float sm_scale, int8_t* q_i8, float* q_scale, float* lse, void* stream);
+int sage_qk_int8_sv_f16_attn_lse_add(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t* v16, void* o,
+                                     int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_s, const float* q_scale,
+                                     const float* k_scale, int out_dtype, int B, int Hq, int Hkv, int Sq, int Skv, int D,
+                                     int is_causal, float* lse, float lse_add_scale, int* status, void* workspace,
+                                     int64_t workspace_bytes, void* stream);
 // Workspace bytes of one launch, as it will plan it: of sage_qk_int8_sv_f16_attn_ws with these sizes and output
 // strides (heads folded where the rule above says so), and of sage_direct_attn_ws.  The public
 // sage_attn_workspace_bytes knows neither the kv heads nor the strides and gives the most that any of them takes.

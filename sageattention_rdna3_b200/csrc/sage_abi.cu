@@ -368,7 +368,7 @@ int launch_attn_streamk(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   sage::MergeParams m;
   m.part_o = p.part_o; m.part_lse = p.part_lse;
   m.o = p.o; m.o_stride_b = p.o_stride_b; m.o_stride_h = p.o_stride_h; m.o_stride_s = p.o_stride_s;
-  m.lse = p.lse;
+  m.lse = p.lse; m.lse_add = p.lse_add; m.lse_add_scale = p.lse_add_scale;
   m.Hq = p.Hq; m.Sq = p.Sq; m.n_q_tiles = p.n_q_tiles;
   m.nkv_full = plan.nkv_full; m.tiles_per_head = plan.tiles_per_head; m.total_tiles = plan.total_tiles;
   m.attn_grid = plan.grid;
@@ -495,6 +495,36 @@ int sage_quant_qk_int8(const sage_strided_t* q, const sage_strided_t* k, const v
   p.k_blocks = static_cast<int>((kg + sage::kKGroupsPerBlock - 1) / sage::kKGroupsPerBlock);
   const int v_blocks = do_v ? v_block_count(B, Hkv, Skv, D) : 0;
   return dispatch_prep(dtype, D, p, v_blocks, static_cast<cudaStream_t>(stream));
+}
+
+int sage_quant_q_mean_dot(const sage_strided_t* q, int dtype, const void* k_mean, int B, int Hq, int Hkv, int Sq, int D,
+                          float sm_scale, int8_t* q_i8, float* q_scale, float* lse, void* stream) {
+  SAGE_REQUIRE(q && q->ptr && k_mean && q_i8 && q_scale && lse, "sage_quant_q_mean_dot: null pointer");
+  SAGE_REQUIRE(dtype == SAGE_DTYPE_F16 || dtype == SAGE_DTYPE_BF16, "sage_quant_q_mean_dot: dtype must be f16 or bf16");
+  SAGE_REQUIRE(D == 64 || D == 128, "sage_quant_q_mean_dot: head_dim must be 64 or 128, got %d", D);
+  SAGE_REQUIRE(B > 0 && Hq > 0 && Hkv > 0 && Hq % Hkv == 0 && Sq >= 0, "sage_quant_q_mean_dot: bad sizes");
+  SAGE_REQUIRE(aligned16(q->ptr) && strides_ok(q) && aligned16(q_i8) && aligned16(k_mean),
+               "sage_quant_q_mean_dot: 16-byte aligned bases and strides of q % 8 == 0");
+  if (Sq == 0) return SAGE_OK;
+  sage::PrepParams p;
+  memset(&p, 0, sizeof(p));
+  p.q = view_of(q);
+  p.q_i8 = q_i8; p.q_scale = q_scale;
+  p.q_mean = k_mean; p.q_mean_dot = lse;
+  p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.Sq = Sq;
+  p.q_groups = (Sq + sage::kQGroupRows - 1) / sage::kQGroupRows;
+  volatile float s = sm_scale;                          // csrc/attn_gfx11.cu:34,1995: one fp32 multiply
+  volatile float l2e = 1.4426950408889634f;
+  p.sm_scale_log2e = s * l2e;
+  const long long qg = static_cast<long long>(B) * Hq * p.q_groups;
+  p.q_blocks = static_cast<int>((qg + sage::kQGroupsPerBlock - 1) / sage::kQGroupsPerBlock);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dtype == SAGE_DTYPE_F16) {
+    return launch(D == 128 ? sage::sage_prep_q_dot_kernel<__half, 128> : sage::sage_prep_q_dot_kernel<__half, 64>, p.q_blocks,
+                  sage::kPrepThreads, 0, st, p);
+  }
+  return launch(D == 128 ? sage::sage_prep_q_dot_kernel<__nv_bfloat16, 128> : sage::sage_prep_q_dot_kernel<__nv_bfloat16, 64>,
+                p.q_blocks, sage::kPrepThreads, 0, st, p);
 }
 
 int sage_prep_smooth_preferred(int B, int Hkv) {
@@ -642,7 +672,8 @@ namespace {
 int attn_int8_impl(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t* v16, void* o, int64_t o_stride_b,
                    int64_t o_stride_h, int64_t o_stride_s, const float* q_scale, const float* k_scale, int out_dtype,
                    int B, int Hq, int Hkv, int Sq, int Skv, int D, int is_causal, float* lse, int32_t* s_dump,
-                   int* status, void* workspace, int64_t workspace_bytes, int n_peers, void* const* peer_o, void* stream);
+                   int* status, void* workspace, int64_t workspace_bytes, int n_peers, void* const* peer_o,
+                   const float* lse_add_scale, void* stream);
 }  // namespace
 
 int sage_qk_int8_sv_f16_attn_ws(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t* v16, void* o,
@@ -651,7 +682,17 @@ int sage_qk_int8_sv_f16_attn_ws(const int8_t* q_i8, const int8_t* k_i8, const sa
                                 int D, int is_causal, float* lse, int32_t* s_dump, int* status, void* workspace,
                                 int64_t workspace_bytes, void* stream) {
   return attn_int8_impl(q_i8, k_i8, v16, o, o_stride_b, o_stride_h, o_stride_s, q_scale, k_scale, out_dtype, B, Hq, Hkv,
-                        Sq, Skv, D, is_causal, lse, s_dump, status, workspace, workspace_bytes, 0, nullptr, stream);
+                        Sq, Skv, D, is_causal, lse, s_dump, status, workspace, workspace_bytes, 0, nullptr, nullptr, stream);
+}
+
+int sage_qk_int8_sv_f16_attn_lse_add(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t* v16, void* o,
+                                     int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_s, const float* q_scale,
+                                     const float* k_scale, int out_dtype, int B, int Hq, int Hkv, int Sq, int Skv, int D,
+                                     int is_causal, float* lse, float lse_add_scale, int* status, void* workspace,
+                                     int64_t workspace_bytes, void* stream) {
+  return attn_int8_impl(q_i8, k_i8, v16, o, o_stride_b, o_stride_h, o_stride_s, q_scale, k_scale, out_dtype, B, Hq, Hkv,
+                        Sq, Skv, D, is_causal, lse, nullptr, status, workspace, workspace_bytes, 0, nullptr, &lse_add_scale,
+                        stream);
 }
 
 int sage_qk_int8_sv_f16_attn_scatter(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t* v16, void* o,
@@ -670,7 +711,7 @@ int sage_qk_int8_sv_f16_attn_scatter(const int8_t* q_i8, const int8_t* k_i8, con
     }
   }
   return attn_int8_impl(q_i8, k_i8, v16, o, o_stride_b, o_stride_h, o_stride_s, q_scale, k_scale, out_dtype, B, Hq, Hkv,
-                        Sq, Skv, D, is_causal, lse, nullptr, status, nullptr, 0, n_peers, peer_o, stream);
+                        Sq, Skv, D, is_causal, lse, nullptr, status, nullptr, 0, n_peers, peer_o, nullptr, stream);
 }
 
 // Mapping of another process's device buffer (one process per GPU on one node): the owner exports
@@ -723,7 +764,8 @@ namespace {
 int attn_int8_impl(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t* v16, void* o, int64_t o_stride_b,
                    int64_t o_stride_h, int64_t o_stride_s, const float* q_scale, const float* k_scale, int out_dtype,
                    int B, int Hq, int Hkv, int Sq, int Skv, int D, int is_causal, float* lse, int32_t* s_dump,
-                   int* status, void* workspace, int64_t workspace_bytes, int n_peers, void* const* peer_o, void* stream) {
+                   int* status, void* workspace, int64_t workspace_bytes, int n_peers, void* const* peer_o,
+                   const float* lse_add_scale, void* stream) {
   SAGE_REQUIRE(q_i8 && v16 && o && q_scale, "sage_qk_int8_sv_f16_attn: null pointer");
   SAGE_REQUIRE(Skv == 0 || (k_i8 && v16->ptr && k_scale), "sage_qk_int8_sv_f16_attn: null pointer");
   SAGE_REQUIRE(out_dtype == SAGE_DTYPE_F16 || out_dtype == SAGE_DTYPE_BF16,
@@ -754,6 +796,10 @@ int attn_int8_impl(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t*
   p.q_fold = fold; p.q_rows = rows_per_head;
   p.q_groups = (rows_per_head + sage::kQGroupRows - 1) / sage::kQGroupRows;
   p.s_dump = s_dump;
+  if (lse != nullptr && lse_add_scale != nullptr) {
+    p.lse_add = 1;
+    p.lse_add_scale = *lse_add_scale;
+  }
   p.n_peers = n_peers;                                  // (the persistent launch does not scatter: plain launch)
   for (int i = 0; i < n_peers; ++i) p.peer_o[i] = peer_o[i];
   if (n_peers > 0 && is_causal) {

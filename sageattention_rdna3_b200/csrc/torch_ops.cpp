@@ -211,11 +211,12 @@ at::Tensor v_to_f16(const at::Tensor& v, int64_t layout) {
 // `lse` (optional, fp32 [B,Hq,Sq]) receives the natural-log sum of exponentials of every row.
 // `peer_ptrs` (optional): device addresses of further copies of `output` (same layout and strides,
 // normally in other GPUs' memory) that the kernel writes as well (sage_qk_int8_sv_f16_attn_scatter).
-at::Tensor qk_int8_sv_f16_attn(const at::Tensor& q_i8, const at::Tensor& k_i8, const at::Tensor& v, at::Tensor& o,
-                               const at::Tensor& q_scale, const at::Tensor& k_scale, int64_t layout,
-                               int64_t is_causal, double /*sm_scale*/, int64_t value_layout,
-                               const c10::optional<at::Tensor>& s_dump, const c10::optional<at::Tensor>& status,
-                               const c10::optional<at::Tensor>& lse, at::OptionalIntArrayRef peer_ptrs) {
+// `lse_add_scale` (not of the operator): sage_qk_int8_sv_f16_attn_lse_add.
+at::Tensor int8_attn(const at::Tensor& q_i8, const at::Tensor& k_i8, const at::Tensor& v, at::Tensor& o,
+                     const at::Tensor& q_scale, const at::Tensor& k_scale, int64_t layout, int64_t is_causal,
+                     int64_t value_layout, const c10::optional<at::Tensor>& s_dump, const c10::optional<at::Tensor>& status,
+                     const c10::optional<at::Tensor>& lse, at::OptionalIntArrayRef peer_ptrs,
+                     const float* lse_add_scale = nullptr) {
   TORCH_CHECK(q_i8.is_cuda() && q_i8.scalar_type() == at::kChar && q_i8.is_contiguous() && q_i8.dim() == 4,
               "query must be a contiguous int8 CUDA tensor [B,Hq,Sq,D]");
   TORCH_CHECK(k_i8.scalar_type() == at::kChar && k_i8.is_contiguous() && k_i8.dim() == 4,
@@ -273,6 +274,15 @@ at::Tensor qk_int8_sv_f16_attn(const at::Tensor& q_i8, const at::Tensor& k_i8, c
   const int64_t ws_bytes = dump_ptr ? 0 : sage_int8_workspace_bytes((int)B, (int)Hq, (int)Hkv, (int)Sq, (int)Skv, (int)D,
                                                                     (int)is_causal, os.stride_h, os.stride_s);
   if (ws_bytes > 0) workspace = at::empty({ws_bytes}, q_i8.options().dtype(at::kByte));
+  if (lse_ptr != nullptr && lse_add_scale != nullptr) {
+    check_rc(sage_qk_int8_sv_f16_attn_lse_add(q_i8.data_ptr<int8_t>(), k_i8.data_ptr<int8_t>(), &vs, o.data_ptr(), os.stride_b,
+                                              os.stride_h, os.stride_s, q_scale.data_ptr<float>(), k_scale.data_ptr<float>(),
+                                              dtype_code(o), (int)B, (int)Hq, (int)Hkv, (int)Sq, (int)Skv, (int)D,
+                                              (int)is_causal, lse_ptr, *lse_add_scale, status_ptr,
+                                              ws_bytes > 0 ? workspace.data_ptr() : nullptr, ws_bytes, current_stream(q_i8)),
+             "qk_int8_sv_f16_attn");
+    return o;
+  }
   check_rc(sage_qk_int8_sv_f16_attn_ws(q_i8.data_ptr<int8_t>(), k_i8.data_ptr<int8_t>(), &vs, o.data_ptr(), os.stride_b,
                                        os.stride_h, os.stride_s, q_scale.data_ptr<float>(),
                                        k_scale.data_ptr<float>(), dtype_code(o), (int)B, (int)Hq, (int)Hkv, (int)Sq,
@@ -280,6 +290,14 @@ at::Tensor qk_int8_sv_f16_attn(const at::Tensor& q_i8, const at::Tensor& k_i8, c
                                        ws_bytes > 0 ? workspace.data_ptr() : nullptr, ws_bytes, current_stream(q_i8)),
            "qk_int8_sv_f16_attn");
   return o;
+}
+
+at::Tensor qk_int8_sv_f16_attn(const at::Tensor& q_i8, const at::Tensor& k_i8, const at::Tensor& v, at::Tensor& o,
+                               const at::Tensor& q_scale, const at::Tensor& k_scale, int64_t layout, int64_t is_causal,
+                               double /*sm_scale*/, int64_t value_layout, const c10::optional<at::Tensor>& s_dump,
+                               const c10::optional<at::Tensor>& status, const c10::optional<at::Tensor>& lse,
+                               at::OptionalIntArrayRef peer_ptrs) {
+  return int8_attn(q_i8, k_i8, v, o, q_scale, k_scale, layout, is_causal, value_layout, s_dump, status, lse, peer_ptrs);
 }
 
 // fp16_attn / bf16_attn(Tensor query, Tensor key, Tensor value, Tensor(a!) output, int tensor_layout,
@@ -401,6 +419,13 @@ std::vector<at::Tensor> sageattn_fwd(const at::Tensor& q, const at::Tensor& k, c
   return {o};
 }
 
+void check_key_mean(const at::Tensor& k_mean, const at::Tensor& q, const Dims& d) {
+  TORCH_CHECK(k_mean.is_contiguous() && k_mean.dim() == 3 && k_mean.size(0) == d.B && k_mean.size(2) == d.D &&
+                  k_mean.size(1) > 0 && d.H % k_mean.size(1) == 0 && k_mean.scalar_type() == q.scalar_type() &&
+                  k_mean.device() == q.device(),
+              "key_mean must be a contiguous [B,Hkv,D] tensor of the input dtype");
+}
+
 // lse_add_q_mean(Tensor(a!) lse, Tensor query, Tensor key_mean, int tensor_layout, float sm_scale) -> ()
 // lse [B,Hq,Sq] += sm_scale * q.mean(k): refers the log-sum-exp of centred keys to the original ones.
 void lse_add_q_mean(at::Tensor& lse, const at::Tensor& q, const at::Tensor& k_mean, int64_t layout, double sm_scale) {
@@ -408,10 +433,7 @@ void lse_add_q_mean(at::Tensor& lse, const at::Tensor& q, const at::Tensor& k_me
   const Dims d = dims_of(q, layout);
   TORCH_CHECK(lse.is_cuda() && lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.numel() == d.B * d.H * d.S,
               "lse must be a contiguous fp32 CUDA tensor [B,Hq,Sq]");
-  TORCH_CHECK(k_mean.is_contiguous() && k_mean.dim() == 3 && k_mean.size(0) == d.B && k_mean.size(2) == d.D &&
-                  k_mean.size(1) > 0 && d.H % k_mean.size(1) == 0 && k_mean.scalar_type() == q.scalar_type() &&
-                  k_mean.device() == q.device(),
-              "key_mean must be a contiguous [B,Hkv,D] tensor of the input dtype");
+  check_key_mean(k_mean, q, d);
   c10::cuda::CUDAGuard guard(q.device());
   const sage_strided_t qs = strided_of(q, layout);
   check_rc(sage_lse_add_q_mean(&qs, dtype_code(q), k_mean.data_ptr(), lse.data_ptr<float>(), (int)d.B, (int)d.H,
@@ -441,16 +463,25 @@ std::vector<at::Tensor> sageattn_kv_fwd(const at::Tensor& q, const at::Tensor& k
   c10::optional<at::Tensor> lse;
   if (want_lse) lse = at::empty({dq.B, dq.H, dq.S}, q.options().dtype(at::kFloat));
   const sage_strided_t qs = strided_of(q, layout);
+  const c10::optional<at::Tensor> st(status), none;
+  if (want_lse && k_mean.has_value()) {
+    // the launches of the other branch, with q . mean taken along by the first and added to the log-sum-exp by the second
+    check_key_mean(*k_mean, q, dq);
+    const float scale = static_cast<float>(sm_scale);
+    check_rc(sage_quant_q_mean_dot(&qs, dtype_code(q), k_mean->data_ptr(), (int)dq.B, (int)dq.H, (int)k_mean->size(1), (int)dq.S,
+                                   (int)dq.D, scale, q_i8.data_ptr<int8_t>(), q_scale.data_ptr<float>(), lse->data_ptr<float>(),
+                                   current_stream(q)),
+             "sageattn_kv_fwd");
+    int8_attn(q_i8, k_i8, v, o, q_scale, k_scale, layout, is_causal, value_layout, none, st, lse, c10::nullopt, &scale);
+    return {o, *lse};
+  }
   sage_strided_t none_k = qs;                            // no keys: only the Q blocks of the launch exist
   check_rc(sage_quant_qk_int8(&qs, &none_k, nullptr, nullptr, nullptr, dtype_code(q), (int)dq.B, (int)dq.H,
                               (int)k_i8.size(1), (int)dq.S, 0, (int)dq.D, static_cast<float>(sm_scale),
                               q_i8.data_ptr<int8_t>(), q_scale.data_ptr<float>(), nullptr, nullptr, current_stream(q)),
            "sageattn_kv_fwd");
-  const c10::optional<at::Tensor> st(status), none;
-  qk_int8_sv_f16_attn(q_i8, k_i8, v, o, q_scale, k_scale, layout, is_causal, sm_scale, value_layout, none, st, lse,
-                      c10::nullopt);
+  int8_attn(q_i8, k_i8, v, o, q_scale, k_scale, layout, is_causal, value_layout, none, st, lse, c10::nullopt);
   if (!want_lse) return {o};
-  if (k_mean.has_value()) lse_add_q_mean(*lse, q, *k_mean, layout, sm_scale);
   return {o, *lse};
 }
 
