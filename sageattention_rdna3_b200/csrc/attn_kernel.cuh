@@ -123,8 +123,8 @@ struct AttnSmem {
   static constexpr int kOffBar = kOffV + kStages * kVBytes;
   // barriers: q_full, o_final, s_full[2], p_full[2], pv_done[2], q_empty, o_free, epi_done (the
   // last three only cycle in the persistent variant), then per stage k_full[], v_full[], k_empty[],
-  // v_empty[]
-  static constexpr int kNumBars = 11 + 4 * kStages;
+  // v_empty[], v_ready[] (the last only where V is converted in shared memory)
+  static constexpr int kNumBars = 11 + 5 * kStages;
   static constexpr int kOffMisc = kOffBar + 8 * kNumBars;   // tmem base (u32), abort flag, fail code
   static constexpr int kTotal = kOffMisc + 16;
 };
@@ -263,7 +263,11 @@ struct SegIter {
 // TMEM, barriers and the K/V ring are set up once per CTA, barrier phases keep counting across
 // segments (kt = KV tiles so far, it = segments so far), and the loads and first Q.K^T of the next
 // segment overlap the epilogue of the previous one.
-template <int D, bool CAUSAL, bool DUMP, bool QKF = false, int KST = 0, bool STREAMK = false>
+// VBF = true (un-quantised, plain launch): V arrives as bf16, and the softmax warps turn each tile into fp16 where it
+// stands, under the Q.K^T of the same tile.  That is one launch instead of two where a call has few items and few
+// tiles (sage_direct_takes_bf16_v); every item converts its own copy of a tile, so with many the conversion ahead of
+// the launch is cheaper.
+template <int D, bool CAUSAL, bool DUMP, bool QKF = false, int KST = 0, bool STREAMK = false, bool VBF = false>
 __global__ void __launch_bounds__(kAttnThreads, 2)
 sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -271,6 +275,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   using L = AttnSmem<D, QKF ? 2 : 1, KST>;
   constexpr int kStages = L::kStages;
   static_assert(!(QKF && DUMP), "the int32 score dump belongs to the quantised variant");
+  static_assert(!VBF || (QKF && !STREAMK), "bf16 V belongs to the plain un-quantised launch");
   extern __shared__ __align__(1024) uint8_t smem[];
 
   const int warp = threadIdx.x >> 5;
@@ -298,6 +303,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint64_t* v_full = bars + 11 + kStages;
   uint64_t* k_empty = bars + 11 + 2 * kStages;
   uint64_t* v_empty = bars + 11 + 3 * kStages;
+  uint64_t* v_ready = bars + 11 + 4 * kStages;   // VBF: the tile has been converted by all 128 softmax threads
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 4);
   int* fail_code = reinterpret_cast<int*>(smem + L::kOffMisc + 8);
@@ -340,6 +346,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       mbar_init(v_full + s, 1);
       mbar_init(k_empty + s, 1);
       mbar_init(v_empty + s, 1);
+      if (VBF) mbar_init(v_ready + s, 128);
     }
     fence_mbar_init();
     fence_proxy_async_smem();
@@ -533,7 +540,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               SAGE_WAIT_OR(p_full + h, t & 1, 5, { ok = false; break; });
-              if (h == 0) SAGE_WAIT_OR(v_full + s, ph, 6, { ok = false; break; });
+              if (h == 0) SAGE_WAIT_OR((VBF ? v_ready : v_full) + s, ph, 6, { ok = false; break; });
               // the first P.V of a segment overwrites O: the previous segment's O must have been read
               if (STREAMK && h == 0 && j == 0 && it > 0) SAGE_WAIT_OR(o_free, (it - 1) & 1, 14, { ok = false; break; });
               tc_fence_after();
@@ -628,6 +635,19 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
       for (int g = 0; g < 4; ++g) cg[g] = QKF ? p.score_scale : __fmul_rn(qs, ks_next[g]);
 
+      if (VBF && h == 0) {
+        const int stage = t % kStages;
+        SAGE_WAIT_OR(v_full + stage, (t / kStages) & 1, 6, { ok = false; break; });
+        uint4* tile = reinterpret_cast<uint4*>(s_v + stage * L::kVBytes) + threadIdx.x;
+#pragma unroll 8
+        for (int i = 0; i < L::kVBytes / (16 * 128); ++i) {
+          const uint4 x = tile[i * 128];
+          auto to_half2 = [](uint32_t w) { return pack_half2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u)); };
+          tile[i * 128] = make_uint4(to_half2(x.x), to_half2(x.y), to_half2(x.z), to_half2(x.w));
+        }
+        fence_proxy_async_smem();                       // the tensor instructions read it through the async proxy
+        mbar_arrive(v_ready + stage);
+      }
       SAGE_WAIT_OR(s_full + h, t & 1, 8, { ok = false; break; });
       tc_fence_after();
       uint32_t sr[2][32];

@@ -52,6 +52,19 @@ static inline int sage_causal_streamk(int64_t heads, int64_t heaviest, double me
   return heaviest >= fewest;
 }
 
+// Whether the un-quantised launch converts a bf16 V itself.  It does so for every item anew, where a launch ahead of it
+// converts each tile once; that launch costs about 3.5 us of host time and 3 us on the GPU.  The conversion of an item's
+// first tile hides under its first Q.K^T; further ones cost 0.3 us (D=128) or half of that.  us per call, launch
+// ahead / inside: 48 items of 1 tile 11.1 / 7.3, 1536 of 1 51.1 / 43.9, D=64 256 of 2 10.7 / 8.6, 160 of 8 20.0 / 19.4, D=128 64 of 4
+// 12.5 / 11.8, 384 of 2 (mean, causal) 19.2 / 20.1, 128 of 8 17.9 / 18.4, 512 of 4 26.5 / 31.1.  So: one tile, or at most
+// 4 (D=128) or 8 tiles per SM.
+static inline int sage_few_v_tiles(int64_t items, int64_t nq, int64_t nkv, int is_causal, int D, int sms) {
+  if (nkv <= 1) return 1;
+  const double mean = is_causal && nq <= nkv ? 0.5 * (double)(nq + 1) : (double)nkv;      // tiles of an item
+  const double per_sm = mean * (items > sms ? (double)items / sms : 1.0);
+  return per_sm <= (D == 128 ? 4.0 : 8.0);
+}
+
 extern "C" {
 // lse[b,h,s] += sm_scale * q[b,h,s,:] . k_mean[b, h / (Hq/Hkv), :], in fp32: refers the log-sum-exp of a
 // launch on centred keys (smooth_k) to the original ones.  lse: contiguous [B,Hq,Sq]; k_mean:
@@ -74,6 +87,12 @@ int sage_qk_int8_sv_f16_attn_lse_add(const int8_t* q_i8, const int8_t* k_i8, con
 int64_t sage_int8_workspace_bytes(int B, int Hq, int Hkv, int Sq, int Skv, int D, int is_causal, int64_t o_stride_h,
                                   int64_t o_stride_s);
 int64_t sage_direct_workspace_bytes(int B, int Hq, int Sq, int Skv, int D, int is_causal);
+// sage_direct_attn on bf16 tensors with V as it is (bf16, converted inside the launch with the rounding of
+// sage_v_to_f16), and whether that is the better way for these sizes.
+int sage_direct_attn_bf16_v(const sage_strided_t* q, const sage_strided_t* k, const sage_strided_t* v, void* o,
+                            int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_s, int B, int Hq, int Hkv, int Sq, int Skv,
+                            int D, int is_causal, float sm_scale, float* lse, int* status, void* stream);
+int sage_direct_takes_bf16_v(int B, int Hq, int Sq, int Skv, int D, int is_causal);
 // Test hook: how many CTAs of plain attention launches have started on each SM of the current device (counted
 // since the library was loaded; synchronises).
 int sage_test_sm_arrivals(unsigned* counts, int n);

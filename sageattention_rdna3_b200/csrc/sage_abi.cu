@@ -331,10 +331,10 @@ int configure_smem(Kernel kern, int smem_bytes, std::atomic<bool>* configured) {
   return SAGE_OK;
 }
 
-template <int D, bool CAUSAL, bool DUMP, bool QKF = false, int KST = 0>
+template <int D, bool CAUSAL, bool DUMP, bool QKF = false, int KST = 0, bool VBF = false>
 int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to,
                 const sage::AttnParams& p, cudaStream_t stream) {
-  auto kern = sage::sage_attn_kernel<D, CAUSAL, DUMP, QKF, KST>;
+  auto kern = sage::sage_attn_kernel<D, CAUSAL, DUMP, QKF, KST, false, VBF>;
   constexpr int kSmem = sage::AttnSmem<D, QKF ? 2 : 1, KST>::kTotal;
   static std::atomic<bool> configured[64];
   int rc = configure_smem(kern, kSmem, configured);
@@ -959,7 +959,7 @@ int check_peers(const char* who, int n_peers, void* const* peer_o, const void* o
 int direct_attn_impl(const sage_strided_t* q, const sage_strided_t* k, const sage_strided_t* v16, void* o,
                      int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_s, int dtype, int B, int Hq, int Hkv,
                      int Sq, int Skv, int D, int is_causal, float sm_scale, float* lse, int* status, void* workspace,
-                     int64_t workspace_bytes, int n_peers, void* const* peer_o, void* stream);
+                     int64_t workspace_bytes, int n_peers, void* const* peer_o, bool v_bf16, void* stream);
 }  // namespace
 
 int sage_direct_attn_ws(const sage_strided_t* q, const sage_strided_t* k, const sage_strided_t* v16, void* o,
@@ -967,7 +967,25 @@ int sage_direct_attn_ws(const sage_strided_t* q, const sage_strided_t* k, const 
                         int Sq, int Skv, int D, int is_causal, float sm_scale, float* lse, int* status,
                         void* workspace, int64_t workspace_bytes, void* stream) {
   return direct_attn_impl(q, k, v16, o, o_stride_b, o_stride_h, o_stride_s, dtype, B, Hq, Hkv, Sq, Skv, D, is_causal,
-                          sm_scale, lse, status, workspace, workspace_bytes, 0, nullptr, stream);
+                          sm_scale, lse, status, workspace, workspace_bytes, 0, nullptr, false, stream);
+}
+
+int sage_direct_attn_bf16_v(const sage_strided_t* q, const sage_strided_t* k, const sage_strided_t* v, void* o,
+                            int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_s, int B, int Hq, int Hkv, int Sq, int Skv,
+                            int D, int is_causal, float sm_scale, float* lse, int* status, void* stream) {
+  return direct_attn_impl(q, k, v, o, o_stride_b, o_stride_h, o_stride_s, SAGE_DTYPE_BF16, B, Hq, Hkv, Sq, Skv, D, is_causal,
+                          sm_scale, lse, status, nullptr, 0, 0, nullptr, true, stream);
+}
+
+int sage_direct_takes_bf16_v(int B, int Hq, int Sq, int Skv, int D, int is_causal) {
+  int sms = 0;
+  StreamKPlan plan;
+  if (B <= 0 || Hq <= 0 || Sq <= 0 || Skv <= 0 || (D != 64 && D != 128) || sm_count(&sms) != SAGE_OK ||
+      plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal) != SAGE_OK || plan.use) {
+    return 0;
+  }
+  const int64_t nq = (Sq + sage::kBlockM - 1) / sage::kBlockM, nkv = (Skv + sage::kBlockN - 1) / sage::kBlockN;
+  return sage_few_v_tiles(nq * B * Hq, nq, nkv, is_causal, D, sms);
 }
 
 int sage_direct_attn_scatter(const sage_strided_t* q, const sage_strided_t* k, const sage_strided_t* v16, void* o,
@@ -977,14 +995,14 @@ int sage_direct_attn_scatter(const sage_strided_t* q, const sage_strided_t* k, c
   const int rc = check_peers("sage_direct_attn_scatter", n_peers, peer_o, o);
   if (rc) return rc;
   return direct_attn_impl(q, k, v16, o, o_stride_b, o_stride_h, o_stride_s, dtype, B, Hq, Hkv, Sq, Skv, D, is_causal,
-                          sm_scale, lse, status, nullptr, 0, n_peers, peer_o, stream);
+                          sm_scale, lse, status, nullptr, 0, n_peers, peer_o, false, stream);
 }
 
 namespace {
 int direct_attn_impl(const sage_strided_t* q, const sage_strided_t* k, const sage_strided_t* v16, void* o,
                      int64_t o_stride_b, int64_t o_stride_h, int64_t o_stride_s, int dtype, int B, int Hq, int Hkv,
                      int Sq, int Skv, int D, int is_causal, float sm_scale, float* lse, int* status, void* workspace,
-                     int64_t workspace_bytes, int n_peers, void* const* peer_o, void* stream) {
+                     int64_t workspace_bytes, int n_peers, void* const* peer_o, bool v_bf16, void* stream) {
   SAGE_REQUIRE(q && q->ptr && v16 && o, "sage_direct_attn: null pointer");
   SAGE_REQUIRE(Skv == 0 || (k && k->ptr && v16->ptr), "sage_direct_attn: null pointer");
   SAGE_REQUIRE(dtype == SAGE_DTYPE_F16 || dtype == SAGE_DTYPE_BF16, "sage_direct_attn: dtype must be f16 or bf16");
@@ -1024,8 +1042,8 @@ int direct_attn_impl(const sage_strided_t* q, const sage_strided_t* k, const sag
   if (rc) return rc;
   rc = encode_strided_16bit(&tk, qk_dt, k_base, D, skv_map, Hkv, B, kk.stride_s, kk.stride_h, kk.stride_b, sage::kBlockN, "k");
   if (rc) return rc;
-  rc = encode_strided_16bit(&tv, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, v_base, D, skv_map, Hkv, B, vv.stride_s, vv.stride_h,
-                            vv.stride_b, sage::kBlockN, "v16");
+  rc = encode_strided_16bit(&tv, v_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, v_base, D, skv_map,
+                            Hkv, B, vv.stride_s, vv.stride_h, vv.stride_b, sage::kBlockN, "v");
   if (rc) return rc;
   rc = encode_strided_16bit(&to, qk_dt, o, D, Sq, Hq, B, o_stride_s, o_stride_h, o_stride_b, 32, "o");
   if (rc) return rc;
@@ -1043,21 +1061,20 @@ int direct_attn_impl(const sage_strided_t* q, const sage_strided_t* k, const sag
                        : launch_attn_streamk<64, false, true>(tq, tk, tv, to, p, plan, workspace, st);
     }
   }
+#define SAGE_LAUNCH(DD, CC, KST)                                                          \
+  (v_bf16 ? launch_attn<DD, CC, false, true, KST, true>(tq, tk, tv, to, p, st)            \
+          : launch_attn<DD, CC, false, true, KST, false>(tq, tk, tv, to, p, st))
   if (D == 128) {
     // A grid that cannot put two CTAs on every SM anyway takes the deeper K/V rings (one CTA per SM).
     int sms = 0;
     rc = sm_count(&sms);
     if (rc) return rc;
     const long long ctas = static_cast<long long>(p.n_q_tiles) * B * Hq;
-    if (ctas <= sms) {
-      return is_causal ? launch_attn<128, true, false, true, 2>(tq, tk, tv, to, p, st)
-                       : launch_attn<128, false, false, true, 2>(tq, tk, tv, to, p, st);
-    }
-    return is_causal ? launch_attn<128, true, false, true>(tq, tk, tv, to, p, st)
-                     : launch_attn<128, false, false, true>(tq, tk, tv, to, p, st);
+    if (ctas <= sms) return is_causal ? SAGE_LAUNCH(128, true, 2) : SAGE_LAUNCH(128, false, 2);
+    return is_causal ? SAGE_LAUNCH(128, true, 0) : SAGE_LAUNCH(128, false, 0);
   }
-  return is_causal ? launch_attn<64, true, false, true>(tq, tk, tv, to, p, st)
-                   : launch_attn<64, false, false, true>(tq, tk, tv, to, p, st);
+  return is_causal ? SAGE_LAUNCH(64, true, 0) : SAGE_LAUNCH(64, false, 0);
+#undef SAGE_LAUNCH
 }
 }  // namespace
 

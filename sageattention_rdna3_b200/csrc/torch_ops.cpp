@@ -310,10 +310,11 @@ at::Tensor qk_int8_sv_f16_attn(const at::Tensor& q_i8, const at::Tensor& k_i8, c
 at::Tensor direct_attn(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, at::Tensor& o, int64_t layout,
                        int64_t value_layout, int64_t is_causal, double sm_scale, int64_t /*bm_sel*/,
                        const c10::optional<at::Tensor>& status, const c10::optional<at::Tensor>& lse,
-                       at::ScalarType want, const char* name, at::OptionalIntArrayRef peer_ptrs = c10::nullopt) {
+                       at::ScalarType want, const char* name, at::OptionalIntArrayRef peer_ptrs = c10::nullopt,
+                       bool bf16_v = false) {
   TORCH_CHECK(q.scalar_type() == want && k.scalar_type() == want && o.scalar_type() == want, name,
               ": query, key and output must be ", want);
-  TORCH_CHECK(v.scalar_type() == at::kHalf, name, ": value must be fp16 (convert bf16 with v_to_f16)");
+  TORCH_CHECK(v.scalar_type() == (bf16_v ? at::kBFloat16 : at::kHalf), name, ": value must be fp16 (convert bf16 with v_to_f16)");
   check_16b(q, "query");
   check_16b(k, "key");
   check_16b(v, "value");
@@ -345,6 +346,13 @@ at::Tensor direct_attn(const at::Tensor& q, const at::Tensor& k, const at::Tenso
                                       (int)dq.B, (int)dq.H, (int)dk.H, (int)dq.S, (int)dk.S, (int)dq.D, (int)is_causal,
                                       (float)sm_scale, lse_ptr, status_ptr, (int)peers.size(), peers.data(),
                                       current_stream(q)),
+             name);
+    return o;
+  }
+  if (bf16_v) {
+    check_rc(sage_direct_attn_bf16_v(&qs, &ks, &vs, o.data_ptr(), os.stride_b, os.stride_h, os.stride_s, (int)dq.B, (int)dq.H,
+                                     (int)dk.H, (int)dq.S, (int)dk.S, (int)dq.D, (int)is_causal, (float)sm_scale, lse_ptr,
+                                     status_ptr, current_stream(q)),
              name);
     return o;
   }
@@ -393,7 +401,11 @@ std::vector<at::Tensor> sageattn_fwd(const at::Tensor& q, const at::Tensor& k, c
   const bool bf16 = q.scalar_type() == at::kBFloat16;
   const c10::optional<at::Tensor> st(status), none;
   if (use_direct) {
-    if (bf16) {
+    const Dims dq = dims_of(q, layout), dv = dims_of(v, layout);
+    if (bf16 && v.scalar_type() == at::kBFloat16 && (!peer_ptrs.has_value() || peer_ptrs->empty()) &&
+        sage_direct_takes_bf16_v((int)dq.B, (int)dq.H, (int)dq.S, (int)dv.S, (int)dq.D, (int)is_causal)) {
+      direct_attn(q, k, v, o, layout, layout, is_causal, sm_scale, 0, st, lse, at::kBFloat16, "bf16_attn", c10::nullopt, true);
+    } else if (bf16) {
       direct_attn(q, k, v_to_f16(v, layout), o, layout, kHND, is_causal, sm_scale, 0, st, lse, at::kBFloat16, "bf16_attn",
                   peer_ptrs);
     } else {
