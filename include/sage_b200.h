@@ -66,9 +66,9 @@ int sage_set_status_mirror(int* host_word);
 int sage_test_set_wait_limit_us(long long us);
 int sage_test_drop_v_load(int on);
 
-/* Launch schedule of the attention entry points that take a workspace: -1 = the library's cost
- * model decides between one CTA per query tile and persistent CTAs (default), 0 = never
- * persistent, 1 = always.  Process-wide; the environment variable SAGE_STREAMK=0|1, read once at
+/* Launch schedule of the attention entry points: -1 = the library decides between one CTA per query
+ * tile, persistent CTAs and persistent CTAs with two query tiles (default), 0 = one CTA per tile, 1 =
+ * persistent CTAs of one tile wherever there is a workspace.  Process-wide; the environment variable SAGE_STREAMK=0|1, read once at
  * the first launch, sets the initial value.  Takes the place of the reference's per-launch
  * environment overrides of its tile choice (csrc/attn_gfx11.cu:2101-2114). */
 int sage_set_streamk(int mode);
@@ -130,10 +130,11 @@ int sage_qk_int8_sv_f16_attn_lse(const int8_t* q_i8, const int8_t* k_i8, const s
 /* Persistent scheduling for problems that do not fill the GPU evenly.
  * No counterpart in the reference.  sage_qk_int8_sv_f16_attn gives every thread block one whole
  * 128-row query tile; a B200 runs 296 of them at a time, so 320 tiles (B=1, H=10, S=4096) take two
- * rounds.  Given a workspace, the _ws entry points cut the work into 296 equal spans of KV-tile
+ * rounds.  Given a workspace, the _ws entry points cut the work into equal spans of KV-tile
  * steps instead, keep partial results (fp32) in the workspace and merge them with a second small
  * kernel; they fall back to the plain launch when that would not pay, when the workspace is NULL
- * or too small, or when s_dump is set.  Results agree with the plain launch to fp32 rounding of
+ * or too small, or when s_dump is set.  (Many short items run on persistent CTAs that take whole items, two query
+ * tiles at a time, with or without a workspace: the same bits as the plain launch.)  Results agree with the plain launch to fp32 rounding of
  * the merge (same int8 products, same softmax).
  * The INT8 launch lets the query heads of a GQA group share query tiles where that gives fewer of them
  * (few queries per head, no causal mask, no s_dump, output rows that run on from one head to the next:

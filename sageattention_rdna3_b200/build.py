@@ -65,6 +65,7 @@ def _run(cmd) -> None:
 
 def build_abi(force: bool = False, verbose: bool = False) -> Path:
     sources = [CSRC / "sage_abi.cu", CSRC / "attn_kernel.cuh", CSRC / "prep_kernels.cuh", CSRC / "merge_kernels.cuh",
+               CSRC / "pair_kernel.cuh",
                CSRC / "ptx_sm100.cuh", CSRC / "internal.h",
                REPO_DIR / "include" / "sage_b200.h"]
     if force or not _up_to_date(LIB_ABI, sources):

@@ -94,6 +94,9 @@ struct AttnParams {
   int sk_nkv_full;              // ceil(Skv / 128)
   float* part_o;                // [gridDim.x][2][128][D] fp32: acc / l of a span that covers part of an item
   float* part_lse;              // [gridDim.x][2][128] fp32: m + log2 l of the same (base 2)
+  int pair_rounds;              // sage_pair_kernel (256 rows in place of 128): whole items per CTA; the steps above are
+                                // those of the items left over, cut into ...
+  int pair_spans;               // ... this many spans
   // Output scatter (plain launch only): every finished tile is also written, with ordinary 16-byte
   // stores, to `n_peers` more buffers that have the layout and strides of `o` - the same slice of the
   // gathered output in the memory of the other GPUs of the node.
@@ -157,6 +160,17 @@ constexpr int kHalfN = kBlockN / 2;      // the softmax works on 64-column halve
 #endif
 constexpr int kMaxSmIds = 1024;
 static __device__ unsigned g_sm_arrivals[kMaxSmIds];
+
+// Item of sage_pair_kernel -> (batch, head) pair and pair of query tiles: heads `head_group` at a time, neighbouring items
+// are neighbouring heads.
+__device__ __forceinline__ void pair_item(int item, int n_heads, int head_group, int n_pairs, int* bh, int* pair) {
+  const int per_group = n_pairs * head_group;
+  const int g_first = item / per_group * head_group;
+  const int g_size = min(head_group, n_heads - g_first);
+  const int within = item - g_first * n_pairs;
+  *pair = within / g_size;
+  *bh = g_first + within - *pair * g_size;
+}
 
 // What one pass of the pipeline works on: KV tiles [kv_lo, kv_lo + n_kv) of one 128-row query tile
 // of one (batch, query head).  slot < 0: the pass covers every KV tile of the item and writes the
@@ -986,6 +1000,8 @@ struct MergeParams {
   long long total_tiles;
   int attn_grid;                // G
   int causal, out_bf16;
+  // after sage_pair_kernel: items of 256 rows in the order of head groups, the first `item_first` of them whole
+  int item_first, n_heads, head_group;
 };
 
 // ROWS: rows of an item per merge CTA, CHUNK: parts whose loads are in flight together.  A thread owns 16-byte pieces of
@@ -1001,19 +1017,22 @@ constexpr int kMergeChunk = 2;
 constexpr int kMergeChunkFew = 8;
 __host__ __device__ constexpr int merge_rows_few(int D) { return 256 * 4 / D; }
 
-template <int D, int ROWS, int CHUNK>
+// ITEM_ROWS: 128, or 256 after sage_pair_kernel.
+template <int D, int ROWS, int CHUNK, int ITEM_ROWS = kBlockM>
 __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams p) {
-  const int item = blockIdx.x / (kBlockM / ROWS);
-  const int row0 = (blockIdx.x - item * (kBlockM / ROWS)) * ROWS;     // first row of this CTA within the item
-  const int bh = item / p.n_q_tiles;
-  const int qt = item - bh * p.n_q_tiles;
+  constexpr bool kPairs = ITEM_ROWS != kBlockM;
+  const int item = blockIdx.x / (ITEM_ROWS / ROWS);
+  const int row0 = (blockIdx.x - item * (ITEM_ROWS / ROWS)) * ROWS;   // first row of this CTA within the item
+  int bh = item / p.n_q_tiles;
+  int qt = item - bh * p.n_q_tiles;
+  if (kPairs) pair_item(p.item_first + item, p.n_heads, p.head_group, p.n_q_tiles, &bh, &qt);
   const int nkv = p.nkv_full;
   const int tiles = p.causal ? min(qt + 1, nkv) : nkv;
   long long before;                                      // steps of this head before query tile qt
   if (!p.causal) before = static_cast<long long>(qt) * nkv;
   else if (qt <= nkv) before = static_cast<long long>(qt) * (qt + 1) / 2;
   else before = static_cast<long long>(nkv) * (nkv + 1) / 2 + static_cast<long long>(qt - nkv) * nkv;
-  const long long start = static_cast<long long>(bh) * p.tiles_per_head + before;
+  const long long start = kPairs ? static_cast<long long>(item) * nkv : static_cast<long long>(bh) * p.tiles_per_head + before;
   const long long end = start + tiles;
   const long long G = p.attn_grid, T = p.total_tiles;
   const int c_first = static_cast<int>(((start + 1) * G - 1) / T);     // CTA that owns step `start`
@@ -1022,15 +1041,15 @@ __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams 
   const int first_slot = ((T * c_first) / G == start) ? 0 : 1;
   grid_dependency_wait();                                // (all of the above is arithmetic on the arguments)
   grid_launch_dependents();
-  if (n_parts == 1 || qt * kBlockM + row0 >= p.Sq) return;
+  if (n_parts == 1 || qt * ITEM_ROWS + row0 >= p.Sq) return;
 
   constexpr int kVecPerRow = D / 4;
   constexpr int kPerThread = ROWS * kVecPerRow / 256;    // float4 per thread: 1, 2 or 4
   constexpr int kRowStep = 256 / kVecPerRow;
   const int r0 = threadIdx.x / kVecPerRow, c4 = threadIdx.x % kVecPerRow;   // rows r0, r0 + kRowStep, ...
   // the first part may be the last segment of its CTA (slot 1), the others are the first of theirs (slot 0)
-  const long long row_first = (static_cast<long long>(c_first) * 2 + first_slot) * kBlockM + row0 + r0;
-  const long long row_other = static_cast<long long>(c_first) * 2 * kBlockM + row0 + r0;
+  const long long row_first = (static_cast<long long>(c_first) * 2 + first_slot) * ITEM_ROWS + row0 + r0;
+  const long long row_other = static_cast<long long>(c_first) * 2 * ITEM_ROWS + row0 + r0;
   float e_max[kPerThread], sum[kPerThread];
   float4 acc[kPerThread];
 #pragma unroll
@@ -1046,7 +1065,7 @@ __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams 
 #pragma unroll
     for (int c = 0; c < CHUNK; ++c) {
       const int k = k0 + c;
-      const long long pr = k == 0 ? row_first : row_other + static_cast<long long>(k) * 2 * kBlockM;
+      const long long pr = k == 0 ? row_first : row_other + static_cast<long long>(k) * 2 * ITEM_ROWS;
 #pragma unroll
       for (int u = 0; u < kPerThread; ++u) {
         e[c][u] = -INFINITY;
@@ -1081,7 +1100,7 @@ __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams 
   const int b = bh / p.Hq, h = bh - b * p.Hq;
 #pragma unroll
   for (int u = 0; u < kPerThread; ++u) {
-    const int row = qt * kBlockM + row0 + r0 + u * kRowStep;
+    const int row = qt * ITEM_ROWS + row0 + r0 + u * kRowStep;
     if (row >= p.Sq) continue;
     const float inv = (sum[u] > 0.0f) ? 1.0f / sum[u] : 0.0f;
     if (p.lse != nullptr && c4 == 0) {

@@ -65,6 +65,39 @@ static inline int sage_few_v_tiles(int64_t items, int64_t nq, int64_t nkv, int i
   return per_sm <= (D == 128 ? 4.0 : 8.0);
 }
 
+// Whether a launch without a causal mask takes two query tiles per CTA (sage_pair_kernel: one persistent CTA per SM, the
+// loads and the first Q.K^T of the next item under the end of the current one).  items: pairs of tiles; nq: tiles per
+// head.  Two kinds of problem gain, measured against the launch taken otherwise (attention launch alone, 900 combinations
+// of items and KV tiles with even nq; then 220 random calls: 1.04 times on average, 0.97 at worst, up to 1.47):
+// - many items of few KV tiles, where the start and end of an item is much of it.  From 5 items per SM: int8 D=128 1.6
+//   times at 2 tiles, 1.2 at 8, 1.1 at 12; D=64 1.4 / 1.1 / 1.05; un-quantised D=128 1.4 / 1.2 / 1.1, D=64 1.2 / 1.05 / 1.0.
+//   With 3 or 4 per SM the last, part-filled round weighs more and the line lies at fewer tiles.
+// - one or two items per SM and a few over, where whole tiles on two CTAs per SM fill the last round badly: 160 items of 32
+//   tiles, int8, D=64 77 -> 73 us, D=128 1.06; 160 of 16, un-quantised, D=128 67 -> 55 us.
+// Long items are no faster this way: the SM's clock rises (the K and V tiles are fetched once for both query tiles), but
+// an item takes more clocks.  An odd number of tiles per head leaves half a pair empty: the rounds are counted in tiles
+// (580 tiles fill two rounds of the launch with a CTA per tile, though they are 300 pairs: 20 heads of 3711 tokens, D=64,
+// 108 us against 130), and with few tiles per head the line lies lower.
+#define SAGE_PAIR_WHOLE_ROUNDS 3          // from here on the items left over are not cut into spans
+static inline int sage_takes_pairs(int64_t items, int64_t nq, int64_t nkv, int D, int qkf, int sms) {
+  const int odd = nq % 2 == 1;
+  if (odd && nq < 9) return 0;
+  const int64_t tiles = odd ? items / ((nq + 1) / 2) * nq : 2 * items;
+  const int64_t rounds = tiles / (2 * sms);
+  if (rounds >= SAGE_PAIR_WHOLE_ROUNDS) {
+    int64_t most;
+    if (!qkf) most = rounds >= 5 ? 12 : (rounds == 4 && D == 64) ? 8 : 4;
+    else if (D == 128) most = rounds >= 5 ? 12 : 0;
+    else most = rounds >= 5 ? 8 : rounds == 4 ? 3 : 1;
+    return nkv <= (odd && nq < 17 ? most / 2 : most);
+  }
+  const double rest = (double)tiles / (2.0 * sms) - (double)rounds;
+  if (rounds < 1 || nkv < 16 || items / sms != rounds) return 0;
+  if (qkf) return D == 128 && rest <= 0.3;
+  if (D == 64) return rest > 0.01 && rest <= 0.2;
+  return rest > 0.0 && rest <= (rounds == 1 ? 0.13 : 0.1) && nkv <= (rounds == 1 ? 40 : 32);
+}
+
 extern "C" {
 // lse[b,h,s] += sm_scale * q[b,h,s,:] . k_mean[b, h / (Hq/Hkv), :], in fp32: refers the log-sum-exp of a
 // launch on centred keys (smooth_k) to the original ones.  lse: contiguous [B,Hq,Sq]; k_mean:

@@ -16,6 +16,7 @@
 #include "attn_kernel.cuh"
 #include "internal.h"
 #include "merge_kernels.cuh"
+#include "pair_kernel.cuh"
 #include "prep_kernels.cuh"
 
 // K-mean scratch of sage_quant_qk_int8_smooth_static: part of the library image, never allocated.
@@ -382,6 +383,66 @@ int launch_attn_streamk(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
                 static_cast<unsigned>(items * (sage::kBlockM / sage::kMergeRows)), 256, 0, stream, m);
 }
 
+// The launch with two query tiles per CTA (pair_kernel.cuh).  `spans` CTAs share the steps of the `rest` items that are
+// left after `rounds` whole ones for every CTA; without partial results (workspace_bytes == 0) a span is a whole item.
+struct PairPlan {
+  bool use = false;
+  int grid = 0, rounds = 0, rest = 0, nkv = 0, spans = 0;
+  size_t workspace_bytes = 0;
+};
+int plan_pairs(PairPlan* plan, int B, int Hq, int Sq, int Skv, int D, int is_causal, bool qkf) {
+  *plan = PairPlan();
+  if (Sq <= 0 || Skv <= 0 || is_causal || streamk_override() >= 0) return SAGE_OK;
+  int sms = 0;
+  const int rc = sm_count(&sms);
+  if (rc) return rc;
+  const long long nq = (Sq + sage::kBlockM - 1) / sage::kBlockM, nkv = (Skv + sage::kBlockN - 1) / sage::kBlockN;
+  const long long items = (nq + 1) / 2 * B * Hq;
+  if (items > 0x3fffffffLL || !sage_takes_pairs(items, nq, nkv, D, qkf ? 1 : 0, sms)) return SAGE_OK;
+  plan->use = true;
+  plan->grid = sms;
+  plan->rounds = static_cast<int>(items / sms);
+  plan->rest = static_cast<int>(items % sms);
+  plan->nkv = static_cast<int>(nkv);
+  const bool cut = plan->rest > 0 && plan->rounds < SAGE_PAIR_WHOLE_ROUNDS;
+  plan->spans = !cut ? plan->rest : static_cast<int>(std::min<long long>(sms, std::max<long long>(1, plan->rest * nkv / 4)));
+  plan->workspace_bytes = cut ? static_cast<size_t>(plan->spans) * 2 * sage::kPairRows * (D + 1) * sizeof(float) : 0;
+  return SAGE_OK;
+}
+
+template <int D, bool QKF>
+int launch_pairs(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, sage::AttnParams p,
+                 const PairPlan& plan, void* workspace, cudaStream_t stream) {
+  constexpr int kSmem = sage::PairSmem<D, QKF>::kTotal;
+  static std::atomic<bool> configured[64];
+  int rc = configure_smem(sage::sage_pair_kernel<D, QKF>, kSmem, configured);
+  if (rc) return rc;
+  p.sk_nkv_full = plan.nkv;
+  p.sk_total_tiles = static_cast<long long>(plan.rest) * plan.nkv;
+  p.pair_rounds = plan.rounds;
+  p.pair_spans = plan.rest > 0 ? plan.spans : 0;
+  p.part_o = static_cast<float*>(workspace);
+  p.part_lse = p.part_o + static_cast<size_t>(plan.spans) * 2 * sage::kPairRows * D;
+  rc = launch(sage::sage_pair_kernel<D, QKF>, static_cast<unsigned>(plan.grid), sage::kPairThreads, kSmem, stream, tq, tk, tv, to, p);
+  if (rc || plan.workspace_bytes == 0) return rc;
+  sage::MergeParams m;
+  memset(&m, 0, sizeof(m));
+  m.part_o = p.part_o; m.part_lse = p.part_lse;
+  m.o = p.o; m.o_stride_b = p.o_stride_b; m.o_stride_h = p.o_stride_h; m.o_stride_s = p.o_stride_s;
+  m.lse = p.lse; m.lse_add = p.lse_add; m.lse_add_scale = p.lse_add_scale;
+  m.Hq = p.Hq; m.Sq = p.Sq; m.n_q_tiles = (p.n_q_tiles + 1) / 2;
+  m.nkv_full = plan.nkv; m.total_tiles = p.sk_total_tiles;
+  m.attn_grid = plan.spans; m.out_bf16 = p.out_bf16;
+  m.item_first = plan.rounds * plan.grid; m.n_heads = p.B * p.Hq; m.head_group = p.head_group;
+  constexpr int kFew = sage::merge_rows_few(D);
+  if (2 * plan.rest <= kFewMergeItems) {
+    return launch(sage::sage_attn_merge_kernel<D, kFew, sage::kMergeChunkFew, sage::kPairRows>,
+                  static_cast<unsigned>(plan.rest * (sage::kPairRows / kFew)), 256, 0, stream, m);
+  }
+  return launch(sage::sage_attn_merge_kernel<D, sage::kMergeRows, sage::kMergeChunk, sage::kPairRows>,
+                static_cast<unsigned>(plan.rest * (sage::kPairRows / sage::kMergeRows)), 256, 0, stream, m);
+}
+
 // Device address of g_static_kmean on the current device, looked up once per device.
 int static_kmean_address(void** out) {
   static void* addr[64] = {};
@@ -647,21 +708,30 @@ int sage_qk_int8_sv_f16_attn_lse(const int8_t* q_i8, const int8_t* k_i8, const s
                                      stream);
 }
 
-int64_t sage_direct_workspace_bytes(int B, int Hq, int Sq, int Skv, int D, int is_causal) {
+namespace {
+int64_t workspace_bytes_of(int B, int Hq, int Sq, int Skv, int D, int is_causal, bool qkf) {
+  PairPlan pairs;
   StreamKPlan plan;
   if (B <= 0 || Hq <= 0 || (D != 64 && D != 128)) return 0;
+  if (plan_pairs(&pairs, B, Hq, Sq, Skv, D, is_causal, qkf) != SAGE_OK) return 0;
+  if (pairs.use) return static_cast<int64_t>(pairs.workspace_bytes);
   if (plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal) != SAGE_OK) return 0;
   return plan.use ? static_cast<int64_t>(plan.workspace_bytes) : 0;
+}
+}  // namespace
+
+int64_t sage_direct_workspace_bytes(int B, int Hq, int Sq, int Skv, int D, int is_causal) {
+  return workspace_bytes_of(B, Hq, Sq, Skv, D, is_causal, true);
 }
 
 int64_t sage_int8_workspace_bytes(int B, int Hq, int Hkv, int Sq, int Skv, int D, int is_causal, int64_t o_stride_h,
                                   int64_t o_stride_s) {
   const int fold = sage_gqa_fold(Hq, Hkv, Sq, o_stride_h, o_stride_s, is_causal);
-  return sage_direct_workspace_bytes(B, Hq / fold, Sq * fold, Skv, D, is_causal);
+  return workspace_bytes_of(B, Hq / fold, Sq * fold, Skv, D, is_causal, false);
 }
 
 int64_t sage_attn_workspace_bytes(int B, int Hq, int Sq, int Skv, int D, int is_causal) {
-  int64_t most = sage_direct_workspace_bytes(B, Hq, Sq, Skv, D, is_causal);
+  int64_t most = std::max(workspace_bytes_of(B, Hq, Sq, Skv, D, is_causal, true), workspace_bytes_of(B, Hq, Sq, Skv, D, is_causal, false));
   for (int hkv = 1; hkv < Hq; ++hkv) {                   // the numbers of kv heads for which heads would be folded
     if (Hq % hkv == 0) most = std::max(most, sage_int8_workspace_bytes(B, Hq, hkv, Sq, Skv, D, is_causal, Sq, 1));
   }
@@ -864,6 +934,17 @@ int attn_int8_impl(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t*
     if (rc) return rc;
   }
   const bool dump = (s_dump != nullptr);
+  if (!dump && n_peers == 0) {
+    PairPlan pairs;
+    int rc = plan_pairs(&pairs, B, Hq, Sq, Skv, D, is_causal, false);
+    if (rc) return rc;
+    if (pairs.use && (pairs.workspace_bytes == 0 ||
+                      (workspace != nullptr && static_cast<size_t>(workspace_bytes) >= pairs.workspace_bytes))) {
+      SAGE_REQUIRE(aligned16(workspace), "sage_qk_int8_sv_f16_attn_ws: workspace must be 16-byte aligned");
+      return D == 128 ? launch_pairs<128, false>(tq, tk, tv, to, p, pairs, workspace, st)
+                      : launch_pairs<64, false>(tq, tk, tv, to, p, pairs, workspace, st);
+    }
+  }
   if (workspace != nullptr && !dump && n_peers == 0) {
     StreamKPlan plan;
     int rc = plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal);
@@ -979,8 +1060,10 @@ int sage_direct_attn_bf16_v(const sage_strided_t* q, const sage_strided_t* k, co
 
 int sage_direct_takes_bf16_v(int B, int Hq, int Sq, int Skv, int D, int is_causal) {
   int sms = 0;
+  PairPlan pairs;
   StreamKPlan plan;
   if (B <= 0 || Hq <= 0 || Sq <= 0 || Skv <= 0 || (D != 64 && D != 128) || sm_count(&sms) != SAGE_OK ||
+      plan_pairs(&pairs, B, Hq, Sq, Skv, D, is_causal, true) != SAGE_OK || pairs.use ||
       plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal) != SAGE_OK || plan.use) {
     return 0;
   }
@@ -1047,6 +1130,17 @@ int direct_attn_impl(const sage_strided_t* q, const sage_strided_t* k, const sag
   if (rc) return rc;
   rc = encode_strided_16bit(&to, qk_dt, o, D, Sq, Hq, B, o_stride_s, o_stride_h, o_stride_b, 32, "o");
   if (rc) return rc;
+  if (n_peers == 0 && !v_bf16) {
+    PairPlan pairs;
+    rc = plan_pairs(&pairs, B, Hq, Sq, Skv, D, is_causal, true);
+    if (rc) return rc;
+    if (pairs.use && (pairs.workspace_bytes == 0 ||
+                      (workspace != nullptr && static_cast<size_t>(workspace_bytes) >= pairs.workspace_bytes))) {
+      SAGE_REQUIRE(aligned16(workspace), "sage_direct_attn_ws: workspace must be 16-byte aligned");
+      return D == 128 ? launch_pairs<128, true>(tq, tk, tv, to, p, pairs, workspace, st)
+                      : launch_pairs<64, true>(tq, tk, tv, to, p, pairs, workspace, st);
+    }
+  }
   if (workspace != nullptr && n_peers == 0) {
     StreamKPlan plan;
     rc = plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal);

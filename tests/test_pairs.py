@@ -1,0 +1,107 @@
+"""The launch with two query tiles per CTA (csrc/pair_kernel.cuh) and the rule that chooses it (csrc/internal.h)."""
+import ctypes
+import subprocess
+
+import pytest
+import torch
+
+import helpers as H
+
+
+def _rule(tmp_path):
+    from sageattention_rdna3_b200.build import CSRC
+    src = tmp_path / "rule.cpp"
+    src.write_text(f'#include "{CSRC}/internal.h"\n'
+                   'extern "C" int rule(long i, long q, long k, int d, int f, int s) { return sage_takes_pairs(i, q, k, d, f, s); }\n')
+    lib = tmp_path / "rule.so"
+    subprocess.run(["g++", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
+    rule = ctypes.CDLL(str(lib)).rule
+    rule.argtypes = [ctypes.c_long] * 3 + [ctypes.c_int] * 3
+    return rule
+
+
+@pytest.mark.parametrize("items,nq,nkv,D,qkf,taken", [
+    (740, 10, 12, 128, 0, 1), (740, 10, 13, 128, 0, 0), (739, 10, 5, 128, 0, 0), (444, 10, 4, 128, 0, 1), (443, 10, 4, 128, 0, 0),
+    (592, 10, 8, 64, 0, 1), (592, 10, 9, 64, 0, 0), (740, 7, 2, 64, 0, 0), (825, 9, 6, 64, 0, 1), (825, 9, 7, 64, 0, 0), (740, 9, 4, 64, 0, 1), (740, 9, 5, 64, 0, 0),
+    (300, 29, 29, 64, 0, 0), (310, 31, 29, 64, 0, 0), (320, 31, 29, 64, 0, 1), (740, 1, 1, 64, 1, 0),
+    (740, 10, 8, 64, 1, 1), (740, 10, 9, 64, 1, 0), (740, 10, 12, 128, 1, 1), (739, 10, 1, 128, 1, 0), (444, 10, 1, 64, 1, 1),
+    (160, 32, 32, 64, 0, 1), (148, 32, 32, 64, 0, 0), (178, 32, 32, 64, 0, 0), (160, 32, 15, 64, 0, 0), (160, 32, 40, 128, 0, 1),
+    (160, 32, 41, 128, 0, 0), (148, 32, 16, 128, 1, 1), (147, 32, 16, 128, 1, 0), (160, 32, 16, 64, 1, 0),
+])
+def test_rule_on_the_host(tmp_path, items, nq, nkv, D, qkf, taken):
+    assert _rule(tmp_path)(items, nq, nkv, D, qkf, 148) == taken
+
+
+def _calls(q, k, v, layout, kernel):
+    from sageattention_rdna3_b200 import sageattn
+    try:
+        H.set_streamk(-1)
+        pairs = sageattn(q, k, v, tensor_layout=layout, return_lse=True, kernel=kernel)
+        H.set_streamk(0)
+        plain = sageattn(q, k, v, tensor_layout=layout, return_lse=True, kernel=kernel)
+    finally:
+        H.set_streamk(-1)
+    return pairs, plain
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel", ["int8", "direct"])
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv,D,dtype,layout", [
+    (2, 93, 31, 1024, 1, 64, torch.float16, "HND"),        # 744 items of one key
+    (1, 149, 149, 1280, 129, 64, torch.bfloat16, "NHD"),   # 745 items, the second KV tile of one key
+    (1, 150, 30, 1150, 200, 128, torch.bfloat16, "HND"),   # nine query tiles: half a pair empty, the last rows ragged
+    (5, 30, 30, 1281, 256, 128, torch.float16, "NHD"),     # a last query tile of one row
+])
+def test_whole_items_equal_the_plain_launch(tmp_path, B, Hq, Hkv, Sq, Skv, D, dtype, layout, kernel):
+    """A row's softmax does not depend on what else its CTA works on: bit for bit the result of one tile per CTA."""
+    nq, nkv = -(-Sq // 128), -(-Skv // 128)
+    items, sms = B * Hq * -(-nq // 2), torch.cuda.get_device_properties(0).multi_processor_count
+    if not _rule(tmp_path)(items, nq, nkv, D, int(kernel == "direct"), sms):
+        pytest.skip("not a problem for pairs on this GPU")
+    q, k, v = (H.randn((B, h, s, D), i, dtype).cuda() for i, (h, s) in enumerate(((Hq, Sq), (Hkv, Skv), (Hkv, Skv))))
+    q[:, :, 5] *= 30                                       # rows whose maximum moves
+    if layout == "NHD":
+        q, k, v = (t.transpose(1, 2).contiguous() for t in (q, k, v))
+    (o, lse), (o2, lse2) = _calls(q, k, v, layout, kernel)
+    assert torch.equal(o, o2) and torch.equal(lse, lse2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv,D,dtype,kernel", [
+    (1, 10, 10, 4096, 4096, 64, torch.float16, "int8"),    # 160 items of 32 tiles on 148 SMs
+    (1, 50, 25, 1500, 2001, 64, torch.bfloat16, "int8"),   # two rounds and 4 over, ragged
+    (3, 53, 53, 250, 2049, 128, torch.bfloat16, "int8"),   # one pair per head, a last KV tile of one key
+    (1, 20, 20, 2048, 2048, 128, torch.float16, "direct"),
+])
+def test_cut_items_match_the_plain_launch(tmp_path, B, Hq, Hkv, Sq, Skv, D, dtype, kernel):
+    """Parts of an item are merged in fp32: apart from the rounding of P to fp16 against another maximum, and one rounding
+    of the output, what the plain launch gives."""
+    nq, nkv = -(-Sq // 128), -(-Skv // 128)
+    items, sms = B * Hq * -(-nq // 2), torch.cuda.get_device_properties(0).multi_processor_count
+    if not _rule(tmp_path)(items, nq, nkv, D, int(kernel == "direct"), sms):
+        pytest.skip("not a problem for pairs on this GPU")
+    q, k, v = (H.randn((B, h, s, D), i, dtype).cuda() for i, (h, s) in enumerate(((Hq, Sq), (Hkv, Skv), (Hkv, Skv))))
+    (o, lse), (o2, lse2) = _calls(q, k, v, "HND", kernel)
+    ulp = 2.0 ** (-10 if dtype == torch.float16 else -7)
+    assert (o.float() - o2.float()).norm() <= ulp * o2.float().norm()
+    assert (lse - lse2).abs().max() <= 1e-5 * lse2.abs().max()
+
+
+@pytest.mark.gpu
+def test_wait_that_cannot_complete_gives_a_status():
+    from sageattention_rdna3_b200 import _native, check_status, sageattn
+    lib = _native.load_abi()
+    q, k, v = (H.randn((1, 149, s, 64), i, torch.float16).cuda() for i, s in enumerate((1280, 128, 128)))
+    good = sageattn(q, k, v, kernel="int8")
+    check_status()
+    try:
+        lib.sage_test_set_wait_limit_us(20000)
+        lib.sage_test_drop_v_load(1)
+        sageattn(q, k, v, kernel="int8")
+        with pytest.raises(RuntimeError, match="device status"):
+            check_status()
+    finally:
+        lib.sage_test_drop_v_load(0)
+        lib.sage_test_set_wait_limit_us(0)
+    assert torch.equal(sageattn(q, k, v, kernel="int8"), good)
+    check_status()
