@@ -51,6 +51,7 @@ def _calls(q, k, v, layout, kernel):
     (1, 149, 149, 1280, 129, 64, torch.bfloat16, "NHD"),   # 745 items, the second KV tile of one key
     (1, 150, 30, 1150, 200, 128, torch.bfloat16, "HND"),   # nine query tiles: half a pair empty, the last rows ragged
     (5, 30, 30, 1281, 256, 128, torch.float16, "NHD"),     # a last query tile of one row
+    (10, 120, 15, 160, 200, 128, torch.bfloat16, "HND"),   # int8: GQA heads folded into ten tiles of 1280 rows
 ])
 def test_whole_items_equal_the_plain_launch(tmp_path, B, Hq, Hkv, Sq, Skv, D, dtype, layout, kernel):
     """A row's softmax does not depend on what else its CTA works on: bit for bit the result of one tile per CTA."""
