@@ -96,7 +96,8 @@ __global__ void __launch_bounds__(kFoldThreads) sage_fold_partial_kernel(const F
 // row, 16 bytes each), adds to one float per row.  One launch in place of the same expression on tensors
 // (copies of q and of the mean in fp32, a batched product, two element-wise steps).  Together with the
 // folding of GQA heads (internal.h): B=4 Hq=32 Hkv=8 Sq=64 against 8192 cached keys, D=128, with a
-// log-sum-exp: 124.6 -> 73.8 us per call.
+// log-sum-exp: 124.6 -> 73.8 us per call.  (Calls against cached keys know the mean before Q is prepared and take the
+// product along there, sage_prep_q_dot_kernel; this launch serves sageattn with smooth_k and a log-sum-exp.)
 template <typename T, int D>
 __global__ void __launch_bounds__(256) sage_lse_mean_kernel(const StridedView q, const T* __restrict__ k_mean,
                                                             float* __restrict__ lse, int Hq, int rep, int Sq,
