@@ -868,7 +868,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
       } else {
         p.part_lse[(static_cast<long long>(blockIdx.x) * 2 + sg.slot) * kBlockM + threadIdx.x] =
-            (l > 0.0f) ? (m_used + log2f(l)) : -INFINITY;
+            (l == 0.0f) ? -INFINITY : (m_used + log2f(l));                    // a sum that is NaN stays NaN
       }
       uint8_t* stage = s_v + warp * ((D / 64) * 4096);
 #pragma unroll
@@ -1081,8 +1081,7 @@ __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams 
       float top = e_max[u];
 #pragma unroll
       for (int c = 0; c < CHUNK; ++c) top = fmaxf(top, e[c][u]);
-      if (top == -INFINITY) continue;                    // no visible keys so far
-      if (k0 > 0) {
+      if (e_max[u] > -INFINITY) {                        // (never in the first round; without keys so far there is nothing to scale)
         const float back = exp2f(e_max[u] - top);
         sum[u] *= back;
         acc[u].x *= back; acc[u].y *= back; acc[u].z *= back; acc[u].w *= back;
@@ -1090,8 +1089,8 @@ __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams 
       e_max[u] = top;
 #pragma unroll
       for (int c = 0; c < CHUNK; ++c) {
-        const float w = exp2f(e[c][u] - top);            // 0 for a part without visible keys
-        if (w == 0.0f) continue;                         // ... which may hold anything
+        if (e[c][u] == -INFINITY) continue;              // no visible keys: may hold anything
+        const float w = exp2f(e[c][u] - top);            // NaN if the part's sum is: the row is NaN then, as in one piece
         sum[u] += w;
         acc[u].x += w * x[c][u].x; acc[u].y += w * x[c][u].y; acc[u].z += w * x[c][u].z; acc[u].w += w * x[c][u].w;
       }
