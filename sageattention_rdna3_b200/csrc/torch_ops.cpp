@@ -378,6 +378,17 @@ at::Tensor bf16_attn(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
                      "bf16_attn");
 }
 
+// Whether the address ranges of two tensors have a byte in common.
+bool spans_meet(const at::Tensor& a, const at::Tensor& b) {
+  auto end = [](const at::Tensor& t) {
+    int64_t last = 0;
+    for (int64_t i = 0; i < t.dim(); ++i) last += (t.size(i) - 1) * t.stride(i);
+    return static_cast<const char*>(t.data_ptr()) + (last + 1) * t.element_size();
+  };
+  if (a.numel() == 0 || b.numel() == 0) return false;
+  return static_cast<const char*>(a.data_ptr()) < end(b) && static_cast<const char*>(b.data_ptr()) < end(a);
+}
+
 // sageattn_fwd(Tensor query, Tensor key, Tensor value, int tensor_layout, int is_causal, float sm_scale,
 //              int smooth_k, int use_direct, Tensor status, Tensor? lse, Tensor? out, int[]? peer_ptrs) -> Tensor[]
 // The whole of the reference's sageattn body after its assertions (sageattention/core.py:96-201) in
@@ -402,7 +413,9 @@ std::vector<at::Tensor> sageattn_fwd(const at::Tensor& q, const at::Tensor& k, c
   const c10::optional<at::Tensor> st(status), none;
   if (use_direct) {
     const Dims dq = dims_of(q, layout), dv = dims_of(v, layout);
+    // (a V that the output overwrites is copied ahead of the launch: its CTAs do not wait for one another)
     if (bf16 && v.scalar_type() == at::kBFloat16 && (!peer_ptrs.has_value() || peer_ptrs->empty()) &&
+        !(out.has_value() && spans_meet(o, v)) &&
         sage_direct_takes_bf16_v((int)dq.B, (int)dq.H, (int)dq.S, (int)dv.S, (int)dq.D, (int)is_causal)) {
       direct_attn(q, k, v, o, layout, layout, is_causal, sm_scale, 0, st, lse, at::kBFloat16, "bf16_attn", c10::nullopt, true);
     } else if (bf16) {

@@ -54,3 +54,21 @@ def test_same_bits_as_with_the_conversion_ahead(B, Hq, Hkv, Sq, Skv, D, causal, 
         H.set_streamk(-1)
     assert torch.equal(o.nan_to_num(7.0), o2.nan_to_num(7.0))
     assert torch.equal(o.isnan(), o2.isnan())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", ["HND", "NHD"])
+@pytest.mark.parametrize("B,heads,S,D", [(1, 8, 128, 64), (2, 48, 117, 128), (1, 20, 512, 128), (1, 18, 1000, 64)])
+def test_output_over_the_values(B, heads, S, D, layout):
+    """`out` may be V, or lie in the same buffer: what a call with few tiles reads and what it writes are kept apart."""
+    from sageattention_rdna3_b200 import sageattn
+    shape = (B, heads, S, D) if layout == "HND" else (B, S, heads, D)
+    q, k, v = (H.randn(shape, i, torch.bfloat16).cuda() for i in range(3))
+    want = sageattn(q, k, v, tensor_layout=layout, kernel="direct")
+    for _ in range(5):
+        o = v.clone()
+        assert torch.equal(sageattn(q, k, o, tensor_layout=layout, kernel="direct", out=o), want)
+    flat = torch.empty(q.numel() + 8 * D, dtype=q.dtype, device="cuda")      # V starts 8 rows behind the output
+    vs, o = flat[8 * D:].view(shape), flat[:q.numel()].view(shape)
+    vs.copy_(v)
+    assert torch.equal(sageattn(q, k, vs, tensor_layout=layout, kernel="direct", out=o), want)
