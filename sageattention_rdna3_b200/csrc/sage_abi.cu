@@ -410,6 +410,12 @@ int plan_pairs(PairPlan* plan, int B, int Hq, int Sq, int Skv, int D, int is_cau
   return SAGE_OK;
 }
 
+// (A call whose workspace is too small or misaligned goes on to the choice between the other two launches, which answer it.)
+bool workspace_serves(const PairPlan& plan, const void* workspace, int64_t bytes) {
+  return plan.workspace_bytes == 0 ||
+         (workspace != nullptr && aligned16(workspace) && bytes > 0 && static_cast<size_t>(bytes) >= plan.workspace_bytes);
+}
+
 template <int D, bool QKF>
 int launch_pairs(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, sage::AttnParams p,
                  const PairPlan& plan, void* workspace, cudaStream_t stream) {
@@ -938,9 +944,7 @@ int attn_int8_impl(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t*
     PairPlan pairs;
     int rc = plan_pairs(&pairs, B, Hq, Sq, Skv, D, is_causal, false);
     if (rc) return rc;
-    if (pairs.use && (pairs.workspace_bytes == 0 ||
-                      (workspace != nullptr && static_cast<size_t>(workspace_bytes) >= pairs.workspace_bytes))) {
-      SAGE_REQUIRE(aligned16(workspace), "sage_qk_int8_sv_f16_attn_ws: workspace must be 16-byte aligned");
+    if (pairs.use && workspace_serves(pairs, workspace, workspace_bytes)) {
       return D == 128 ? launch_pairs<128, false>(tq, tk, tv, to, p, pairs, workspace, st)
                       : launch_pairs<64, false>(tq, tk, tv, to, p, pairs, workspace, st);
     }
@@ -1134,9 +1138,7 @@ int direct_attn_impl(const sage_strided_t* q, const sage_strided_t* k, const sag
     PairPlan pairs;
     rc = plan_pairs(&pairs, B, Hq, Sq, Skv, D, is_causal, true);
     if (rc) return rc;
-    if (pairs.use && (pairs.workspace_bytes == 0 ||
-                      (workspace != nullptr && static_cast<size_t>(workspace_bytes) >= pairs.workspace_bytes))) {
-      SAGE_REQUIRE(aligned16(workspace), "sage_direct_attn_ws: workspace must be 16-byte aligned");
+    if (pairs.use && workspace_serves(pairs, workspace, workspace_bytes)) {
       return D == 128 ? launch_pairs<128, true>(tq, tk, tv, to, p, pairs, workspace, st)
                       : launch_pairs<64, true>(tq, tk, tv, to, p, pairs, workspace, st);
     }

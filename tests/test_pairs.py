@@ -106,3 +106,30 @@ def test_wait_that_cannot_complete_gives_a_status():
         lib.sage_test_set_wait_limit_us(0)
     assert torch.equal(sageattn(q, k, v, kernel="int8"), good)
     check_status()
+
+
+@pytest.mark.gpu
+def test_workspace_that_is_not_needed_may_be_anywhere():
+    """Whole items use no workspace, and the plain launch that would take them otherwise does not look at it either."""
+    from sageattention_rdna3_b200 import _native
+    lib = _native.load_abi()
+    n_heads, Sq, Skv, D = 259, 512, 256, 64
+    q, k, v = (H.randn((1, n_heads, s, D), i, torch.float16).cuda() for i, s in enumerate((Sq, Skv, Skv)))
+    q_i8, q_scale, k_i8, k_scale, _ = H.abi_quant(q, k, None, "HND", D ** -0.5)
+    ws = torch.zeros(64 << 20, dtype=torch.uint8, device="cuda")
+    outs = []
+    for schedule, offset in ((0, 0), (-1, 0), (-1, 4)):
+        o, vs, status = torch.empty_like(q), H.strided(v, "HND"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        H.set_streamk(schedule)
+        try:
+            rc = lib.sage_qk_int8_sv_f16_attn_ws(q_i8.data_ptr(), k_i8.data_ptr(), ctypes.byref(vs), o.data_ptr(), n_heads * Sq * D,
+                                                 Sq * D, D, q_scale.data_ptr(), k_scale.data_ptr(), 0, 1, n_heads, n_heads, Sq, Skv,
+                                                 D, 0, None, None, status.data_ptr(), ws.data_ptr() + offset, ws.numel() - 16,
+                                                 H._stream())
+        finally:
+            H.set_streamk(-1)
+        assert rc == 0, lib.sage_last_error()
+        assert int(status.item()) == 0
+        outs.append(o)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    assert not ws.any()
