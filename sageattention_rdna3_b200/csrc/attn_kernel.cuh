@@ -184,6 +184,9 @@ struct Segment {
 // within a group the heaviest (last) query tiles go first and neighbouring CTAs are neighbouring
 // heads.  The CTAs resident at any moment then read the K/V of a few heads only (they stay in L2),
 // and the query heads of one KV head (GQA) run together.  The last group of a causal launch is larger.
+// (Divisions of unsigned numbers, one for both the tile and the head: the map stands ahead of the first load of
+// every item.  With signed ones 512 items of 4 tiles, un-quantised, D=128, take 24.08 instead of 23.47 us, 320 items of
+// one tile, D=64, 10.89 instead of 10.77.)
 // STREAMK = true: the KV-tile steps of all items, in (batch, head, query tile) order, form one line
 // of sk_total_tiles steps; CTA c owns steps [c*T/G, (c+1)*T/G) and walks through the items they
 // belong to: the tail of one item, whole items, the head of another.  All CTAs get the same amount
@@ -220,15 +223,15 @@ struct SegIter {
       int g_first = p.tail_first, g_size = p.tail_size, within = blockIdx.x;
       if (!CAUSAL || within < p.tail_block) {
         const int per_group = p.n_q_tiles * p.head_group;
-        const int group = within / per_group;
+        const int group = static_cast<unsigned>(within) / static_cast<unsigned>(per_group);
         g_first = group * p.head_group;
         g_size = CAUSAL ? p.head_group : min(p.head_group, p.B * p.Hq - g_first);
         within -= group * per_group;
       } else {
         within -= p.tail_block;
       }
-      const int qt = p.light_first ? within / g_size : p.n_q_tiles - 1 - within / g_size;
-      fill(s, g_first + within % g_size, qt);
+      const int row = static_cast<unsigned>(within) / static_cast<unsigned>(g_size);
+      fill(s, g_first + within - row * g_size, p.light_first ? row : p.n_q_tiles - 1 - row);
       const int kv_limit = CAUSAL ? min(s.q_base + kBlockM, p.Skv) : p.Skv;   // csrc/attn_gfx11.cu:502
       s.kv_lo = 0;
       s.n_kv = (kv_limit + kBlockN - 1) / kBlockN;
