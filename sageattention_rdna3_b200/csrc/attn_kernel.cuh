@@ -871,7 +871,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
       } else {
         p.part_lse[(static_cast<long long>(blockIdx.x) * 2 + sg.slot) * kBlockM + threadIdx.x] =
-            (l == 0.0f) ? -INFINITY : (m_used + log2f(l));                    // a sum that is NaN stays NaN
+            (l > 0.0f) ? (m_used + log2f(l)) : (l == 0.0f) ? -INFINITY : INFINITY;   // (the merge: a sum that is NaN)
       }
       uint8_t* stage = s_v + warp * ((D / 64) * 4096);
 #pragma unroll
@@ -987,6 +987,9 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 // skipped.  For the others, part k (k = 0 .. n-1) holds o_k = acc_k / l_k and e_k = m_k + log2 l_k
 // over its share of the keys, and
 //     o = sum_k 2^(e_k - E) o_k / sum_k 2^(e_k - E),   E = max_k e_k,   lse = (E + log2 sum) ln 2.
+// A part without visible keys has e_k = -inf and o_k = 0.  What is not a number goes the way it goes in an item of one
+// piece: a part whose l_k is NaN has e_k = +inf, which makes the row NaN (inf - inf), and no part is left out for a
+// weight of 0 (0 * NaN of V is NaN there too).
 // Which CTA holds which part follows from the same arithmetic as SegIter: CTA c owns the steps
 // [c*T/G, (c+1)*T/G); a part that starts at the first step of its CTA is in slot 0, the other
 // possible part of a CTA (its last segment) in slot 1.
@@ -1084,7 +1087,8 @@ __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams 
       float top = e_max[u];
 #pragma unroll
       for (int c = 0; c < CHUNK; ++c) top = fmaxf(top, e[c][u]);
-      if (e_max[u] > -INFINITY) {                        // (never in the first round; without keys so far there is nothing to scale)
+      if (top == -INFINITY) continue;                    // no visible keys so far
+      if (k0 > 0) {
         const float back = exp2f(e_max[u] - top);
         sum[u] *= back;
         acc[u].x *= back; acc[u].y *= back; acc[u].z *= back; acc[u].w *= back;
@@ -1092,8 +1096,7 @@ __global__ void __launch_bounds__(256) sage_attn_merge_kernel(const MergeParams 
       e_max[u] = top;
 #pragma unroll
       for (int c = 0; c < CHUNK; ++c) {
-        if (e[c][u] == -INFINITY) continue;              // no visible keys: may hold anything
-        const float w = exp2f(e[c][u] - top);            // NaN if the part's sum is: the row is NaN then, as in one piece
+        const float w = exp2f(e[c][u] - top);
         sum[u] += w;
         acc[u].x += w * x[c][u].x; acc[u].y += w * x[c][u].y; acc[u].z += w * x[c][u].z; acc[u].w += w * x[c][u].w;
       }

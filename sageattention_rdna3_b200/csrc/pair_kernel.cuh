@@ -456,7 +456,7 @@ sage_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           *dst = p.lse_add ? fmaf(p.lse_add_scale, *dst, lse) : lse;
         }
       } else {
-        p.part_lse[part_row] = (l == 0.0f) ? -INFINITY : (m_used + log2f(l));      // a sum that is NaN stays NaN
+        p.part_lse[part_row] = (l > 0.0f) ? (m_used + log2f(l)) : (l == 0.0f) ? -INFINITY : INFINITY;
       }
       uint8_t* stage = smem + L::kOffStage + warp * 4096;
 #pragma unroll
