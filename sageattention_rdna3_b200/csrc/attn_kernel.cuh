@@ -230,8 +230,9 @@ struct SegIter {
       } else {
         within -= p.tail_block;
       }
-      const int row = static_cast<unsigned>(within) / static_cast<unsigned>(g_size);
-      fill(s, g_first + within - row * g_size, p.light_first ? row : p.n_q_tiles - 1 - row);
+      const int up = static_cast<unsigned>(within) / static_cast<unsigned>(g_size);
+      const int qt = p.light_first ? up : p.n_q_tiles - 1 - up;
+      fill(s, g_first + within - up * g_size, qt);
       const int kv_limit = CAUSAL ? min(s.q_base + kBlockM, p.Skv) : p.Skv;   // csrc/attn_gfx11.cu:502
       s.kv_lo = 0;
       s.n_kv = (kv_limit + kBlockN - 1) / kBlockN;
