@@ -69,18 +69,29 @@ static inline int sage_few_v_tiles(int64_t items, int64_t nq, int64_t nkv, int i
 
 // Whether a launch without a causal mask takes two query tiles per CTA (sage_pair_kernel: one persistent CTA per SM, the
 // loads and the first Q.K^T of the next item under the end of the current one).  items: pairs of tiles; nq: tiles per
-// head.  Two kinds of problem gain, measured against the launch taken otherwise (attention launch alone, 900 combinations
-// of items and KV tiles with even nq; then 220 random calls: 1.04 times on average, 0.97 at worst, up to 1.47):
-// - many items of few KV tiles, where the start and end of an item is much of it.  From 5 items per SM: int8 D=128 1.6
-//   times at 2 tiles, 1.2 at 8, 1.1 at 12; D=64 1.4 / 1.1 / 1.05; un-quantised D=128 1.4 / 1.2 / 1.1, D=64 1.2 / 1.05 / 1.0.
-//   With 3 or 4 per SM the last, part-filled round weighs more and the line lies at fewer tiles.
-// - one or two items per SM and a few over, where whole tiles on two CTAs per SM fill the last round badly: 160 items of 32
-//   tiles, int8, D=64 77 -> 73 us, D=128 1.06; 160 of 16, un-quantised, D=128 67 -> 55 us.
+// head.  Figures: time of the attention launch that is taken otherwise (with its merge) over that of this one, from 1600
+// combinations of heads, query tiles and KV tiles.  Two kinds of problem gain:
+// - many items of few KV tiles, where the start and end of an item is much of it.  From 5 rounds (of 2 tiles per SM) on,
+//   at 2 / 4 / 8 / 12 KV tiles: int8 D=128 1.54 / 1.41 / 1.26 / 1.15 (13: 0.95-1.1), D=64 1.39 / 1.31 / 1.16 / 1.08
+//   (beyond, 1.03-1.08); un-quantised D=128 1.39 / 1.38 / 1.26 / 1.10, D=64 1.22 / 1.19 / 1.04 / 1.01.  (Otherwise means
+//   persistent CTAs of one tile for most of these.  Against one CTA per tile it is 1.0-1.2 up to 4 tiles and 0.9-1.0 at 8.)
+//   With 3 or 4 rounds the last, part-filled one weighs more: int8 at 4 / 8 tiles D=64 1.14 / 0.95 (3 rounds), 1.30 / 1.15
+//   (4), D=128 0.98 / 0.98 and 1.05 / 0.97; un-quantised D=64 at 1 / 2 / 4 tiles 1.19 / 1.04 / 0.92 and at 3 / 8 1.27 / 1.04 (4),
+//   D=128 0.90-1.2 without an order.  Where they are badly filled: sage_pairs_fill.
+// - one or two rounds and a few items over, whose steps are cut into spans, where whole tiles on two CTAs per SM fill
+//   the last round badly.  int8, D=64, with 0.06 to 0.2 of a round over and up to 96 KV tiles 1.00-1.13 (160 items of 32
+//   tiles 77.5 -> 73.5 us); with less over 0.95-1.02 (spans of one tile each, and more to merge), longer items 0.99-1.01.
+//   D=128 where the items over are cut into whole spans of 4 tiles 1.03-1.18; where spans reach over the end of an item
+//   0.96-1.06, and 0.93-0.96 of what the launch taken otherwise is now; measured up to 0.13 or 0.1 of a round and 40 or 32
+//   tiles.  Un-quantised, D=128, up to 0.3 of a round 1.01-1.30.
 // Long items are no faster this way: the SM's clock rises (the K and V tiles are fetched once for both query tiles), but
 // an item takes more clocks.  An odd number of tiles per head leaves half a pair empty: the rounds are counted in tiles
 // (580 tiles fill two rounds of the launch with a CTA per tile, though they are 300 pairs: 20 heads of 3711 tokens, D=64,
-// 108 us against 130), and with few tiles per head the line lies lower.
+// 108 us against 130).  Cut launches, int8, D=64: 0.92-1.00 with more KV tiles than query tiles or less than 0.07 of a round
+// over, else 1.00-1.16.  Whole items: with 9 to 15 tiles per head the line lies at half as many KV tiles (from 5 rounds on,
+// int8 D=64, 3 / 13 tiles 1.22 / 0.97; un-quantised 4 / 12 1.19 / 0.97), with fewer than 9 they are not taken (0.8-1.4 at 1 to 4 tiles).
 #define SAGE_PAIR_WHOLE_ROUNDS 3          // from here on the items left over are not cut into spans
+#define SAGE_PAIR_SPAN_TILES 4            // fewest KV tiles of a span, unless the items left over have fewer
 static inline int sage_takes_pairs(int64_t items, int64_t nq, int64_t nkv, int D, int qkf, int sms) {
   const int odd = nq % 2 == 1;
   if (odd && nq < 9) return 0;
@@ -96,8 +107,24 @@ static inline int sage_takes_pairs(int64_t items, int64_t nq, int64_t nkv, int D
   const double rest = (double)tiles / (2.0 * sms) - (double)rounds;
   if (rounds < 1 || nkv < 16 || items / sms != rounds) return 0;
   if (qkf) return D == 128 && rest <= 0.3;
-  if (D == 64) return rest > 0.01 && rest <= 0.2;
+  if (D == 64) return rest > (odd ? 0.07 : 0.06) && rest <= 0.2 && nkv <= (odd && nq < 96 ? nq : 96);
+  if (nkv % SAGE_PAIR_SPAN_TILES != 0 || items % sms * (nkv / SAGE_PAIR_SPAN_TILES) > sms) return 0;
   return rest > 0.0 && rest <= (rounds == 1 ? 0.13 : 0.1) && nkv <= (rounds == 1 ? 40 : 32);
+}
+
+// Whether whole pairs fill their rounds well enough, the last of which takes as long as the others, where the other choice
+// is one CTA per tile.  Idle slots cost in proportion to the KV tiles of an item.  int8, 3 and 4 rounds, KV tiles times the
+// idle share against the speed of one CTA per tile: D=128 up to 0.3 1.02-1.16, 0.35-0.44 1.01-1.02, 0.45-0.7 0.98-1.00 (one
+// KV tile, 1.04-1.16 throughout, stays below), 0.8-0.95 0.94-0.99; D=64 0.4-0.5 0.99-1.09, 0.66 0.97, 0.95 0.91.  Where half pairs
+// (an odd number of tiles per head) bring one round more than the tiles have, 0.2-0.25 1.04-1.16, 0.26-0.33 0.93-0.99, 0.5
+// 0.95.  More rounds and un-quantised calls (sage_takes_pairs) are faster as pairs all the same.
+static inline int sage_pairs_fill(int64_t items, int64_t nq, int64_t nkv, int D, int qkf, int sms) {
+  const int64_t tiles = items / ((nq + 1) / 2) * nq;
+  const int64_t rounds = tiles / (2 * sms), pair_rounds = (items + sms - 1) / sms;
+  if (qkf || rounds < SAGE_PAIR_WHOLE_ROUNDS || rounds >= 5) return 1;
+  const double idle = 2.0 * (double)sms * (double)pair_rounds / (double)tiles - 1.0;
+  const int one_more = pair_rounds > (tiles + 2 * sms - 1) / (2 * sms);
+  return (double)nkv * idle <= (one_more ? 0.25 : D == 64 ? 0.5 : 0.44);
 }
 
 extern "C" {

@@ -399,13 +399,18 @@ int plan_pairs(PairPlan* plan, int B, int Hq, int Sq, int Skv, int D, int is_cau
   const long long nq = (Sq + sage::kBlockM - 1) / sage::kBlockM, nkv = (Skv + sage::kBlockN - 1) / sage::kBlockN;
   const long long items = (nq + 1) / 2 * B * Hq;
   if (items > 0x3fffffffLL || !sage_takes_pairs(items, nq, nkv, D, qkf ? 1 : 0, sms)) return SAGE_OK;
+  if (!sage_pairs_fill(items, nq, nkv, D, qkf ? 1 : 0, sms)) {
+    StreamKPlan other;
+    const int other_rc = plan_streamk(&other, B, Hq, Sq, Skv, D, is_causal);
+    if (other_rc || !other.use) return other_rc;         // (against persistent CTAs of one tile they gain 1.2-1.5 times)
+  }
   plan->use = true;
   plan->grid = sms;
   plan->rounds = static_cast<int>(items / sms);
   plan->rest = static_cast<int>(items % sms);
   plan->nkv = static_cast<int>(nkv);
   const bool cut = plan->rest > 0 && plan->rounds < SAGE_PAIR_WHOLE_ROUNDS;
-  plan->spans = !cut ? plan->rest : static_cast<int>(std::min<long long>(sms, std::max<long long>(1, plan->rest * nkv / 4)));
+  plan->spans = !cut ? plan->rest : static_cast<int>(std::min<long long>(sms, std::max<long long>(1, plan->rest * nkv / SAGE_PAIR_SPAN_TILES)));
   plan->workspace_bytes = cut ? static_cast<size_t>(plan->spans) * 2 * sage::kPairRows * (D + 1) * sizeof(float) : 0;
   return SAGE_OK;
 }
