@@ -28,7 +28,7 @@ def _rule(tmp_path, name="sage_takes_pairs"):
     (160, 32, 32, 64, 0, 1), (148, 32, 32, 64, 0, 0), (178, 32, 32, 64, 0, 0), (160, 32, 15, 64, 0, 0), (160, 32, 40, 128, 0, 1),
     (160, 32, 41, 128, 0, 0), (148, 32, 16, 128, 1, 1), (147, 32, 16, 128, 1, 0), (160, 32, 16, 64, 1, 0),
     # cut launches: half pairs, a round hardly begun, long items, spans that reach over the end of an item
-    (320, 31, 29, 64, 0, 1), (320, 31, 32, 64, 0, 0), (180, 71, 71, 64, 0, 1), (180, 71, 72, 64, 0, 0), (170, 19, 19, 64, 0, 0), (152, 16, 21, 64, 0, 0),
+    (320, 31, 29, 64, 0, 1), (320, 31, 32, 64, 0, 0), (180, 71, 71, 64, 0, 1), (180, 71, 72, 64, 0, 0), (170, 19, 19, 64, 0, 1), (170, 19, 20, 64, 0, 0), (152, 16, 21, 64, 0, 0),
     (157, 2, 21, 64, 0, 1), (160, 32, 96, 64, 0, 1), (160, 32, 97, 64, 0, 0), (165, 129, 96, 64, 0, 0), (320, 128, 128, 64, 0, 0),
     (160, 32, 36, 128, 0, 1), (160, 32, 37, 128, 0, 0), (167, 2, 28, 128, 0, 1), (167, 2, 32, 128, 0, 0), (168, 55, 20, 128, 0, 1),
     (170, 19, 40, 128, 0, 0), (162, 18, 20, 128, 1, 1), (365, 9, 60, 128, 1, 1),
