@@ -1,4 +1,5 @@
-"""Items that are cut into parts and merged hand on what is not a number, like items in one piece."""
+"""Persistent launches against the plain one where only some items, or none, are cut: what is not a number, and items of
+one tile."""
 import pytest
 import torch
 
@@ -35,3 +36,22 @@ def test_not_a_number_is_where_it_is_in_one_piece(B, Hq, Sq, Skv, D, kernel, sch
     # elsewhere: one rounding of the output, and that of P against other maxima (fp16)
     ok = want.isfinite() & got.isfinite()
     assert (got[ok].float() - want[ok].float()).norm() <= 2.0 ** -10 * want[ok].float().norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel", ["int8", "direct"])
+@pytest.mark.parametrize("B,heads,Sq,Skv,D,causal", [(1, 1, 1, 1, 64, False), (2, 301, 300, 128, 128, False), (1, 300, 128, 77, 64, True)])
+def test_items_of_one_tile(B, heads, Sq, Skv, D, causal, kernel):
+    """One tile per item: nothing is cut, and every output is written without a merge."""
+    from sageattention_rdna3_b200 import check_status, sageattn
+    q, k, v = (H.randn((B, heads, s, D), i, torch.bfloat16).cuda() for i, s in enumerate((Sq, Skv, Skv)))
+    outs = []
+    for schedule in (0, 1):
+        try:
+            H.set_streamk(schedule)
+            out = torch.full_like(q, float("nan"))
+            outs.append(sageattn(q, k, v, is_causal=causal, kernel=kernel, return_lse=True, out=out))
+        finally:
+            H.set_streamk(-1)
+    check_status()
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
