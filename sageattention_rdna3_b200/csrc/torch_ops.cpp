@@ -400,6 +400,8 @@ std::vector<at::Tensor> sageattn_fwd(const at::Tensor& q, const at::Tensor& k, c
                                      int64_t is_causal, double sm_scale, int64_t smooth_k, int64_t use_direct,
                                      const at::Tensor& status, const c10::optional<at::Tensor>& lse,
                                      const c10::optional<at::Tensor>& out, at::OptionalIntArrayRef peer_ptrs) {
+  // (also for the choice of the launch, which asks for the number of SMs)
+  c10::cuda::CUDAGuard guard(q.device());
   at::Tensor o;
   if (out.has_value()) {
     TORCH_CHECK(out->sizes() == q.sizes() && out->scalar_type() == q.scalar_type() && out->device() == q.device(),
@@ -427,7 +429,6 @@ std::vector<at::Tensor> sageattn_fwd(const at::Tensor& q, const at::Tensor& k, c
     return {o};
   }
   const Dims dk_all = dims_of(k, layout);
-  c10::cuda::CUDAGuard guard(q.device());
   if (smooth_k && sage_prep_smooth_preferred((int)dk_all.B, (int)dk_all.H)) {
     // few heads: one launch for the mean and the quantisation against it
     std::vector<at::Tensor> parts =
