@@ -37,19 +37,26 @@ static inline int sage_tail_group_first(int n_heads, int head_group, int n_q_til
 }
 
 // Persistent or plain launch under a causal mask.  The plain launch takes as long as its heaviest item, a CTA by
-// itself for most of the time (5 us + 1.15 us per KV tile), or as all items together on all slots (two CTAs per SM,
-// 6 us + 2 us per tile and slot), whichever is more; its items come heaviest first, so the two do not add up.  The
-// persistent launch cuts the steps into equal spans, but a span in the light end of a head is many items of one to
-// a few tiles, each with its own start and end, and that span is the last to finish.  So it pays only where the heaviest item alone
-// is far above the mean: few heads, long ones.  Plain / persistent, us, attention launch with its merge (n heads of
-// t tiles): D=64 1 of 64 79 / 36, 2 of 48 61 / 37, 4 of 40 58 / 52, 5 of 24 38 / 40, 14 of 24 38 / 58; D=128 1 of 64 80 / 45,
-// 2 of 40 53 / 40, 3 of 32 47 / 43, 4 of 40 55 / 60, 10 of 24 37 / 62; un-quantised within a few per cent of that.
+// itself for most of the time (5 us + 1.15 us per KV tile, 1.4 times that where running maxima move), or as all items
+// together on all slots (two CTAs per SM, 6 us + 2 us per tile and slot), whichever is more; its items come heaviest first,
+// so the two do not add up.  The persistent launch cuts the steps into equal spans, but a span in the light end of a head
+// is many items of one to a few tiles, each with its own start and end, and that span is the last to finish.  So it pays only where
+// the heaviest item alone is far above the mean: few heads, long ones.  Time of the persistent launch with its merge over
+// that of the plain one, N(0,1) inputs / x20 outliers, ranges over 8 to 48 tiles in the heaviest item:
+//   D=64, int8: 1 head 0.40-0.71 / 0.35-0.59, 3 0.69-0.88 / 0.59-0.74, 5 0.90-1.04 / 0.73-0.91, 6 from 14 to 32 tiles
+//   0.95-1.05 / 0.81-0.92, 8 0.99-1.29 / 0.82-1.25; un-quantised 5 0.87-0.99 / 0.67-0.85, 8 from 16 to 28 tiles 0.95-1.05 /
+//   0.81-0.86, 10 1.14-1.36 / 0.90-1.21;
+//   D=128: 1 head 0.50-0.78 / 0.41-0.61, 2 0.68-0.88 / 0.53-0.68, 3 0.83-1.10 / 0.67-0.86, 4 from 20 tiles on 0.93-1.04 / 0.71-0.86,
+//   below 0.92-1.19 / 0.71-0.93, 5 1.08-1.30 / 0.86-1.00.
+// With 64 tiles 4 heads, D=64, 0.97 / 0.94, 5 heads 1.09 / 1.07: the heaviest item is less than 2.2 times the mean.
 // heads: (batch, query head) pairs; heaviest: KV tiles of the heaviest item; mean_steps: KV tiles per CTA of the
 // persistent launch.
-static inline int sage_causal_streamk(int64_t heads, int64_t heaviest, double mean_steps, int D) {
-  if (heads > (D == 64 ? 4 : 3) || heaviest < 2.2 * mean_steps) return 0;
-  const int fewest = D == 64 ? (heads <= 2 ? 8 : 20) : (heads == 1 ? 8 : heads == 2 ? 24 : 32);
-  return heaviest >= fewest;
+static inline int sage_causal_streamk(int64_t heads, int64_t heaviest, double mean_steps, int D, int qkf = 0) {
+  if (heaviest < 8 || heaviest < 2.2 * mean_steps) return 0;
+  if (D == 128) return heads <= 3 || (heads == 4 && heaviest >= 20);
+  if (heads <= 5) return 1;
+  if (heads == 6) return heaviest >= 14 && heaviest >= 2.8 * mean_steps;
+  return qkf && heads <= 8 && heaviest >= 16 && heaviest >= 2.5 * mean_steps;
 }
 
 // Whether the un-quantised launch converts a bf16 V itself.  It does so for every item anew, where a launch ahead of it

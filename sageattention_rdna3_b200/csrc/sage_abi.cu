@@ -268,7 +268,7 @@ struct StreamKPlan {
   size_t workspace_bytes = 0;
 };
 
-int plan_streamk(StreamKPlan* plan, int B, int Hq, int Sq, int Skv, int D, int is_causal) {
+int plan_streamk(StreamKPlan* plan, int B, int Hq, int Sq, int Skv, int D, int is_causal, bool qkf) {
   *plan = StreamKPlan();
   if (Sq <= 0 || Skv <= 0) return SAGE_OK;
   const int forced = streamk_override();
@@ -289,7 +289,7 @@ int plan_streamk(StreamKPlan* plan, int B, int Hq, int Sq, int Skv, int D, int i
   const long long grid = total < slots ? total : slots;
   bool use;
   if (is_causal) {
-    use = sage_causal_streamk(static_cast<long long>(B) * Hq, std::min(nq, nkv), static_cast<double>(total) / grid, D) != 0;
+    use = sage_causal_streamk(static_cast<long long>(B) * Hq, std::min(nq, nkv), static_cast<double>(total) / grid, D, qkf ? 1 : 0) != 0;
   } else {
     // Makespans in KV-tile steps of a CTA that shares its SM with another one.  Plain launch: full
     // waves of `slots` items, then a tail wave that runs about 1.4x faster per CTA if it leaves every
@@ -403,7 +403,7 @@ int plan_pairs(PairPlan* plan, int B, int Hq, int Sq, int Skv, int D, int is_cau
   if (items > 0x3fffffffLL || !sage_takes_pairs(items, nq, nkv, D, qkf ? 1 : 0, sms)) return SAGE_OK;
   if (!sage_pairs_fill(items, nq, nkv, D, qkf ? 1 : 0, sms)) {
     StreamKPlan other;
-    const int other_rc = plan_streamk(&other, B, Hq, Sq, Skv, D, is_causal);
+    const int other_rc = plan_streamk(&other, B, Hq, Sq, Skv, D, is_causal, qkf);
     if (other_rc || !other.use) return other_rc;         // (against persistent CTAs of one tile they gain 1.2-1.5 times)
   }
   plan->use = true;
@@ -728,7 +728,7 @@ int64_t workspace_bytes_of(int B, int Hq, int Sq, int Skv, int D, int is_causal,
   if (B <= 0 || Hq <= 0 || (D != 64 && D != 128)) return 0;
   if (plan_pairs(&pairs, B, Hq, Sq, Skv, D, is_causal, qkf) != SAGE_OK) return 0;
   if (pairs.use) return static_cast<int64_t>(pairs.workspace_bytes);
-  if (plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal) != SAGE_OK) return 0;
+  if (plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal, qkf) != SAGE_OK) return 0;
   return plan.use ? static_cast<int64_t>(plan.workspace_bytes) : 0;
 }
 }  // namespace
@@ -958,7 +958,7 @@ int attn_int8_impl(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t*
   }
   if (workspace != nullptr && !dump && n_peers == 0) {
     StreamKPlan plan;
-    int rc = plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal);
+    int rc = plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal, false);
     if (rc) return rc;
     if (plan.use && static_cast<size_t>(workspace_bytes) >= plan.workspace_bytes) {
       SAGE_REQUIRE(aligned16(workspace), "sage_qk_int8_sv_f16_attn_ws: workspace must be 16-byte aligned");
@@ -1075,7 +1075,7 @@ int sage_direct_takes_bf16_v(int B, int Hq, int Sq, int Skv, int D, int is_causa
   StreamKPlan plan;
   if (B <= 0 || Hq <= 0 || Sq <= 0 || Skv <= 0 || (D != 64 && D != 128) || sm_count(&sms) != SAGE_OK ||
       plan_pairs(&pairs, B, Hq, Sq, Skv, D, is_causal, true) != SAGE_OK || pairs.use ||
-      plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal) != SAGE_OK || plan.use) {
+      plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal, true) != SAGE_OK || plan.use) {
     return 0;
   }
   const int64_t nq = (Sq + sage::kBlockM - 1) / sage::kBlockM, nkv = (Skv + sage::kBlockN - 1) / sage::kBlockN;
@@ -1152,7 +1152,7 @@ int direct_attn_impl(const sage_strided_t* q, const sage_strided_t* k, const sag
   }
   if (workspace != nullptr && n_peers == 0) {
     StreamKPlan plan;
-    rc = plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal);
+    rc = plan_streamk(&plan, B, Hq, Sq, Skv, D, is_causal, true);
     if (rc) return rc;
     if (plan.use && static_cast<size_t>(workspace_bytes) >= plan.workspace_bytes) {
       SAGE_REQUIRE(aligned16(workspace), "sage_direct_attn_ws: workspace must be 16-byte aligned");

@@ -45,8 +45,10 @@ def test_every_item_has_one_block(tmp_path):
 
 
 @pytest.mark.parametrize("heads,tiles,D,persistent", [
-    (1, 7, 64, 0), (1, 8, 64, 1), (4, 19, 64, 0), (4, 20, 64, 1), (5, 40, 64, 0), (4, 96, 64, 0),
-    (1, 7, 128, 0), (1, 8, 128, 1), (2, 23, 128, 0), (2, 24, 128, 1), (3, 31, 128, 0), (3, 32, 128, 1), (4, 40, 128, 0),
+    (1, 7, 64, 0), (1, 8, 64, 1), (4, 7, 64, 0), (4, 8, 64, 1), (5, 40, 64, 1), (5, 64, 64, 0), (4, 96, 64, 0), (6, 13, 64, 0),
+    (6, 32, 64, 1), (6, 40, 64, 0), (8, 20, 64, 0),
+    (1, 7, 128, 0), (1, 8, 128, 1), (2, 7, 128, 0), (2, 8, 128, 1), (3, 32, 128, 1), (4, 19, 128, 0), (4, 20, 128, 1), (4, 40, 128, 1),
+    (5, 40, 128, 0),
     (10, 24, 128, 0), (64, 64, 128, 0),
 ])
 def test_few_long_causal_heads_are_cut_into_spans(tmp_path, heads, tiles, D, persistent):
