@@ -64,10 +64,12 @@ static inline int sage_causal_streamk(int64_t heads, int64_t heaviest, double me
 // first tile hides under its first Q.K^T; further ones cost 0.3 us (D=128) or half of that.  us per call, launch
 // ahead / inside: 48 items of 1 tile 11.1 / 7.3, 1536 of 1 51.1 / 43.9, D=64 256 of 2 10.7 / 8.6, 160 of 8 20.0 / 19.4, D=128 64 of 4
 // 12.5 / 11.8, 384 of 2 (mean, causal) 19.2 / 20.1, 128 of 8 17.9 / 18.4, 512 of 4 26.5 / 31.1.  So: one tile, or at most
-// 4 (D=128) or 8 tiles per SM.  With D=128 and more items than SMs the rings hold one tile, and the conversion stands
+// 4 (D=128) or 8 tiles per SM.  One tile, D=128, stays ahead where there are more than 4 items per SM and several of them to
+// a tile of V: 1080 items, 45 to a head, 28.1 / 29.1, 1200, 6 to a head, 33.3 / 34.4, but 1100, one to a head, 37.4 / 31.9, and
+// 576, 24 to a head, 16.2 / 16.3.  With D=128 and more items than SMs the rings hold one tile, and the conversion stands
 // between each load and its use: 160 causal items of 3 (mean) 18.0 / 21.7.
 static inline int sage_few_v_tiles(int64_t items, int64_t nq, int64_t nkv, int is_causal, int D, int sms) {
-  if (nkv <= 1) return 1;
+  if (nkv <= 1) return D == 64 || items <= 4 * (int64_t)sms || nq <= 3;
   if (D == 128 && items > sms) return 0;
   const double mean = is_causal && nq <= nkv ? 0.5 * (double)(nq + 1) : (double)nkv;      // tiles of an item
   const double per_sm = mean * (items > sms ? (double)items / sms : 1.0);

@@ -9,7 +9,8 @@ import helpers as H
 
 
 @pytest.mark.parametrize("items,nq,nkv,causal,D,inside", [
-    (48, 1, 1, 0, 128, 1), (100000, 64, 1, 0, 128, 1), (64, 4, 4, 0, 128, 1), (64, 4, 5, 0, 128, 0), (149, 1, 2, 0, 128, 0), (148, 2, 2, 0, 128, 1),
+    (48, 1, 1, 0, 128, 1), (100000, 64, 1, 0, 128, 0), (100000, 64, 1, 0, 64, 1), (592, 64, 1, 0, 128, 1), (593, 64, 1, 0, 128, 0),
+    (1000, 3, 1, 0, 128, 1),  (64, 4, 4, 0, 128, 1), (64, 4, 5, 0, 128, 0), (149, 1, 2, 0, 128, 0), (148, 2, 2, 0, 128, 1),
     (112, 7, 7, 1, 128, 1), (128, 8, 8, 1, 128, 0), (148, 8, 8, 0, 64, 1), (149, 8, 8, 0, 64, 0), (20, 3, 20, 1, 64, 1),
 ])
 def test_rule_on_the_host(tmp_path, items, nq, nkv, causal, D, inside):
