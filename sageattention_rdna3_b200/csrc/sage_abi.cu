@@ -448,12 +448,14 @@ int launch_pairs(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap
   m.attn_grid = plan.spans; m.out_bf16 = p.out_bf16;
   m.item_first = plan.rounds * plan.grid; m.n_heads = p.B * p.Hq; m.head_group = p.head_group;
   constexpr int kFew = sage::merge_rows_few(D);
-  if (2 * plan.rest <= kFewMergeItems) {
-    return launch(sage::sage_attn_merge_kernel<D, kFew, sage::kMergeChunkFew, sage::kPairRows>,
-                  static_cast<unsigned>(plan.rest * (sage::kPairRows / kFew)), 256, 0, stream, m);
+  if constexpr (D == 128 && QKF) {                       // the others have at most 33 items left over (sage_takes_pairs)
+    if (2 * plan.rest > kFewMergeItems) {
+      return launch(sage::sage_attn_merge_kernel<D, sage::kMergeRows, sage::kMergeChunk, sage::kPairRows>,
+                    static_cast<unsigned>(plan.rest * (sage::kPairRows / sage::kMergeRows)), 256, 0, stream, m);
+    }
   }
-  return launch(sage::sage_attn_merge_kernel<D, sage::kMergeRows, sage::kMergeChunk, sage::kPairRows>,
-                static_cast<unsigned>(plan.rest * (sage::kPairRows / sage::kMergeRows)), 256, 0, stream, m);
+  return launch(sage::sage_attn_merge_kernel<D, kFew, sage::kMergeChunkFew, sage::kPairRows>,
+                static_cast<unsigned>(plan.rest * (sage::kPairRows / kFew)), 256, 0, stream, m);
 }
 
 // Device address of g_static_kmean on the current device, looked up once per device.
