@@ -128,5 +128,6 @@ def abi_attn(q_i8, k_i8, v16, v_layout, q_scale, k_scale, out_dtype, out_layout,
 
 
 def set_streamk(mode):
-    """Launch schedule of the attention kernels: -1 cost model, 0 plain, 1 persistent (sage_set_streamk)."""
+    """Launch schedule of the attention kernels (sage_set_streamk): -1 the library's choice, 0 one CTA per query tile,
+    1 persistent CTAs of one tile.  0 and 1 switch pairs of query tiles off."""
     assert _native.load_abi().sage_set_streamk(int(mode)) == 0

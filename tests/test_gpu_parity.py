@@ -5,6 +5,7 @@ Bars: int8 values, fp32 scales, K mean and int32 Q.K^T are bit-exact; the attent
 cosine >= 0.999 and relative L1 <= 1e-2 against the oracle, and stays inside the reference's own
 gates against fp32 SDPA (cosine > 0.99 fp16 / 0.98 bf16, max-abs < 0.35; test_sageattn_rdna3.py:39-53).
 """
+import ctypes
 import os
 import sys
 
@@ -661,15 +662,23 @@ def test_persistent_launch_matches_plain_launch_and_oracle(dev, monkeypatch, cas
 
 
 def test_scheduler_choices_for_known_shapes(dev, monkeypatch):
-    """sage_attn_workspace_bytes > 0 means the persistent launch will be used.  The choices below are
-    the measured ones: 320 items of 32 steps (the reference's headline shape) and the 4-head VAE shape gain from
-    it, one exact wave, two nearly full waves and the 4096-item B=2 H=32 S=8192 causal shape do not."""
+    """sage_attn_workspace_bytes > 0 means that items are cut, by one of the kernels at least.  The choices below are
+    the measured ones: 320 items of 32 steps (the reference's headline shape; its INT8 call as 160 pairs of query tiles, the
+    12 left over in 96 spans) and the 4-head VAE shape gain from it, one exact wave, two nearly full waves and the 4096-item
+    B=2 H=32 S=8192 causal shape do not."""
     H.set_streamk(-1)
     lib = H._native.load_abi()
     torch.cuda.set_device(dev)
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     want = lambda B, Hq, Sq, Skv, D, causal: lib.sage_attn_workspace_bytes(B, Hq, Sq, Skv, D, causal)
     assert want(1, 10, 4096, 4096, 64, 0) == 2 * sms * 2 * 128 * (64 + 1) * 4
+    int8 = lib.sage_int8_workspace_bytes
+    int8.argtypes, int8.restype = [ctypes.c_int] * 7 + [ctypes.c_int64] * 2, ctypes.c_int64
+    if sms == 148:
+        assert int8(1, 10, 10, 4096, 4096, 64, 0, 4096 * 64, 64) == 96 * 2 * 256 * (64 + 1) * 4
+    direct = lib.sage_direct_workspace_bytes
+    direct.argtypes, direct.restype = [ctypes.c_int] * 6, ctypes.c_int64
+    assert direct(1, 10, 4096, 4096, 64, 0) == 2 * sms * 2 * 128 * (64 + 1) * 4
     assert want(1, 4, 16384, 16384, 128, 0) == 2 * sms * 2 * 128 * (128 + 1) * 4
     assert want(1, 1, 8192, 8192, 128, 1) > 0                 # one causal head: 64 very unequal items
     assert want(1, 2 * sms // 8, 1024, 4096, 128, 0) == 0     # exactly one wave of items

@@ -6,15 +6,7 @@ import torch
 import helpers as H
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("schedule", [0, 1])
-@pytest.mark.parametrize("layout,causal", [("HND", False), ("NHD", False), ("HND", True)])
-@pytest.mark.parametrize("B,Hkv,rep,Sq,Skv,D,dtype", [
-    (1, 1, 1, 1, 16, 64, torch.float16),          # one row
-    (2, 2, 4, 31, 300, 128, torch.bfloat16),      # folded heads (HND), a group that is not full
-    (1, 3, 2, 200, 1500, 64, torch.bfloat16),     # two query tiles, the second ragged
-])
-def test_equals_the_sum_of_two_launches(B, Hkv, rep, Sq, Skv, D, dtype, layout, causal, schedule):
+def _compare(B, Hkv, rep, Sq, Skv, D, dtype, layout, causal, schedule):
     """Bit for bit what the launch without a mean and sage_lse_add_q_mean behind it give."""
     from sageattention_rdna3_b200 import _native, quantize_kv, sageattn_quantized_kv
     ops = _native.load_ops()
@@ -35,3 +27,29 @@ def test_equals_the_sum_of_two_launches(B, Hkv, rep, Sq, Skv, D, dtype, layout, 
     ops.lse_add_q_mean(lse2, q, kv.k_mean, lay, D ** -0.5)
     assert torch.equal(o, o2)
     assert torch.equal(lse, lse2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("schedule", [0, 1])
+@pytest.mark.parametrize("layout,causal", [("HND", False), ("NHD", False), ("HND", True)])
+@pytest.mark.parametrize("B,Hkv,rep,Sq,Skv,D,dtype", [
+    (1, 1, 1, 1, 16, 64, torch.float16),          # one row
+    (2, 2, 4, 31, 300, 128, torch.bfloat16),      # folded heads (HND), a group that is not full
+    (1, 3, 2, 200, 1500, 64, torch.bfloat16),     # two query tiles, the second ragged
+])
+def test_equals_the_sum_of_two_launches(B, Hkv, rep, Sq, Skv, D, dtype, layout, causal, schedule):
+    _compare(B, Hkv, rep, Sq, Skv, D, dtype, layout, causal, schedule)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,Hkv,rep,Sq,Skv,D,dtype,layout", [
+    (1, 149, 1, 1280, 129, 64, torch.bfloat16, "NHD"),     # whole items
+    (10, 15, 8, 160, 200, 128, torch.bfloat16, "HND"),     # whole items of folded heads
+    (1, 10, 1, 4096, 4000, 64, torch.float16, "HND"),      # cut and merged, the last KV tile ragged
+    (1, 83, 2, 250, 3500, 128, torch.float16, "NHD"),      # the same, the second query tile ragged too
+])
+def test_pairs_of_query_tiles(tmp_path, B, Hkv, rep, Sq, Skv, D, dtype, layout):
+    """... and where two query tiles share a CTA, which schedules 0 and 1 exclude."""
+    from test_pairs import _assert_pairs
+    _assert_pairs(tmp_path, B, Hkv * rep, Hkv, Sq, Skv, D, "int8", layout)
+    _compare(B, Hkv, rep, Sq, Skv, D, dtype, layout, False, -1)

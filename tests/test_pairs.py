@@ -46,6 +46,16 @@ def test_rounds_that_are_badly_filled(tmp_path, items, nq, nkv, D, qkf, filled):
     assert _rule(tmp_path, "sage_pairs_fill")(items, nq, nkv, D, qkf, 148) == filled
 
 
+def _assert_pairs(tmp_path, B, Hq, Hkv, Sq, Skv, D, kernel, layout):
+    """The call is one that the rule takes (int8: with the heads of a GQA group folded where that is done)."""
+    sms, rep = torch.cuda.get_device_properties(0).multi_processor_count, Hq // Hkv
+    if kernel == "int8" and layout == "HND" and -(-rep * Sq // 128) < rep * -(-Sq // 128):
+        Hq, Sq = Hkv, rep * Sq
+    nq, nkv = -(-Sq // 128), -(-Skv // 128)
+    case = B * Hq * -(-nq // 2), nq, nkv, D, int(kernel == "direct"), sms
+    assert sms != 148 or (_rule(tmp_path)(*case) and _rule(tmp_path, "sage_pairs_fill")(*case))
+
+
 def _calls(q, k, v, layout, kernel):
     from sageattention_rdna3_b200 import sageattn
     try:
@@ -63,16 +73,13 @@ def _calls(q, k, v, layout, kernel):
 @pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv,D,dtype,layout", [
     (2, 93, 31, 1024, 1, 64, torch.float16, "HND"),        # 744 items of one key
     (1, 149, 149, 1280, 129, 64, torch.bfloat16, "NHD"),   # 745 items, the second KV tile of one key
-    (1, 150, 30, 1150, 200, 128, torch.bfloat16, "HND"),   # nine query tiles: half a pair empty, the last rows ragged
+    (1, 165, 33, 1150, 200, 128, torch.bfloat16, "HND"),   # nine query tiles: half a pair empty, the last rows ragged
     (5, 30, 30, 1281, 256, 128, torch.float16, "NHD"),     # a last query tile of one row
     (10, 120, 15, 160, 200, 128, torch.bfloat16, "HND"),   # int8: GQA heads folded into ten tiles of 1280 rows
 ])
 def test_whole_items_equal_the_plain_launch(tmp_path, B, Hq, Hkv, Sq, Skv, D, dtype, layout, kernel):
     """A row's softmax does not depend on what else its CTA works on: bit for bit the result of one tile per CTA."""
-    nq, nkv = -(-Sq // 128), -(-Skv // 128)
-    items, sms = B * Hq * -(-nq // 2), torch.cuda.get_device_properties(0).multi_processor_count
-    if not _rule(tmp_path)(items, nq, nkv, D, int(kernel == "direct"), sms):
-        pytest.skip("not a problem for pairs on this GPU")
+    _assert_pairs(tmp_path, B, Hq, Hkv, Sq, Skv, D, kernel, layout)
     q, k, v = (H.randn((B, h, s, D), i, dtype).cuda() for i, (h, s) in enumerate(((Hq, Sq), (Hkv, Skv), (Hkv, Skv))))
     q[:, :, 5] *= 30                                       # rows whose maximum moves
     if layout == "NHD":
@@ -94,9 +101,7 @@ def test_cut_items_match_the_plain_launch(tmp_path, B, Hq, Hkv, Sq, Skv, D, dtyp
     the output in either, and P rounded to fp16 against another maximum in either (2^-11 of its value, or 2^-25 of
     its largest value for what is below fp16's normal numbers)."""
     from sageattention_rdna3_b200 import sageattn
-    nq, nkv = -(-Sq // 128), -(-Skv // 128)
-    items, sms = B * Hq * -(-nq // 2), torch.cuda.get_device_properties(0).multi_processor_count
-    assert sms != 148 or _rule(tmp_path)(items, nq, nkv, D, int(kernel == "direct"), sms)
+    _assert_pairs(tmp_path, B, Hq, Hkv, Sq, Skv, D, kernel, "HND")
     q, k, v = (H.randn((B, h, s, D), i, dtype) for i, (h, s) in enumerate(((Hq, Sq), (Hkv, Skv), (Hkv, Skv))))
     q[:, :, 3::31] *= 12                                   # rows whose maximum moves
     k[:, :, Skv // 2 :: 97] *= 3                           # ... by more in the later parts
@@ -158,3 +163,62 @@ def test_workspace_that_is_not_needed_may_be_anywhere():
         outs.append(o)
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
     assert not ws.any()
+
+
+CASES_IN_USE = [
+    (149, 1280, 129, 64, torch.bfloat16, "int8"),          # whole items
+    (10, 4096, 4096, 64, torch.float16, "int8"),           # cut
+    (20, 2048, 2048, 128, torch.float16, "direct"),        # cut
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,Sq,Skv,D,dtype,kernel", CASES_IN_USE)
+def test_slices_of_larger_tensors(tmp_path, heads, Sq, Skv, D, dtype, kernel):
+    """Q, K, V and the output as slices: the same bits as for contiguous tensors, and nothing written beside the output."""
+    from sageattention_rdna3_b200 import sageattn
+    _assert_pairs(tmp_path, 1, heads, heads, Sq, Skv, D, kernel, "NHD")
+    qs = H.randn((1, Sq, heads, 2 * D), 0, dtype).cuda()
+    kvs = H.randn((1, Skv, 2, heads, D + 8), 1, dtype).cuda()
+    q, k, v = qs[..., D:], kvs[:, :, 0, :, 8:], kvs[:, :, 1, :, :D]
+    buf = torch.full((1, Sq + 3, heads, D + 16), 7.0, dtype=dtype, device="cuda")
+    out = buf[:, 2:-1, :, 8:-8]
+    sageattn(q, k, v, tensor_layout="NHD", kernel=kernel, out=out)
+    want = sageattn(q.contiguous(), k.contiguous(), v.contiguous(), tensor_layout="NHD", kernel=kernel)
+    assert torch.equal(out, want)
+    out.fill_(7.0)
+    assert (buf == 7.0).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,Sq,Skv,D,dtype,kernel", CASES_IN_USE)
+def test_captured_and_on_two_streams(tmp_path, heads, Sq, Skv, D, dtype, kernel):
+    """A captured call replayed on new inputs, and calls in flight on two streams, each with its workspace."""
+    from sageattention_rdna3_b200 import check_status, sageattn
+    _assert_pairs(tmp_path, 1, heads, heads, Sq, Skv, D, kernel, "HND")
+    sets = [[H.randn((1, heads, s, D), 3 * n + i, dtype).cuda() for i, s in enumerate((Sq, Skv, Skv))] for n in range(2)]
+    want = [sageattn(*t, kernel=kernel) for t in sets]
+    mine = [t.clone() for t in sets[0]]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        sageattn(*mine, kernel=kernel)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = sageattn(*mine, kernel=kernel)
+    for n in (0, 1):
+        for a, b in zip(mine, sets[n]):
+            a.copy_(b)
+        graph.replay()
+        assert torch.equal(out, want[n])
+    streams = [torch.cuda.Stream() for _ in sets]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(4):
+        for n, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                got[n].append(sageattn(*sets[n], kernel=kernel))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want[n]) for n in (0, 1) for o in got[n])
+    check_status()

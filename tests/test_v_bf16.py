@@ -10,7 +10,7 @@ import helpers as H
 
 @pytest.mark.parametrize("items,nq,nkv,causal,D,inside", [
     (48, 1, 1, 0, 128, 1), (100000, 64, 1, 0, 128, 0), (100000, 64, 1, 0, 64, 1), (592, 64, 1, 0, 128, 1), (593, 64, 1, 0, 128, 0),
-    (1000, 3, 1, 0, 128, 1),  (64, 4, 4, 0, 128, 1), (64, 4, 5, 0, 128, 0), (149, 1, 2, 0, 128, 0), (148, 2, 2, 0, 128, 1),
+    (1000, 3, 1, 0, 128, 1), (64, 4, 4, 0, 128, 1), (64, 4, 5, 0, 128, 0), (149, 1, 2, 0, 128, 0), (148, 2, 2, 0, 128, 1),
     (112, 7, 7, 1, 128, 1), (128, 8, 8, 1, 128, 0), (148, 8, 8, 0, 64, 1), (149, 8, 8, 0, 64, 0), (20, 3, 20, 1, 64, 1),
 ])
 def test_rule_on_the_host(tmp_path, items, nq, nkv, causal, D, inside):
@@ -35,26 +35,32 @@ def test_rule_on_the_host(tmp_path, items, nq, nkv, causal, D, inside):
     (1, 8, 2, 500, 500, 128, True),
     (1, 3, 3, 900, 1000, 64, False),              # eight tiles, rings of two
     (1, 160, 160, 128, 60, 128, False),           # more items than SMs: rings of one tile
+    (1, 160, 160, 100, 100, 128, True),
+    (1, 8, 8, 700, 700, 64, True),
+    (1, 160, 32, 200, 300, 64, False),            # two items per SM
 ])
 def test_same_bits_as_with_the_conversion_ahead(B, Hq, Hkv, Sq, Skv, D, causal, layout):
     """The conversion is the same rounding wherever it is done, infinities and what overflows fp16 included."""
     from sageattention_rdna3_b200 import _native, sageattn
     ops = _native.load_ops()
+    assert torch.cuda.get_device_properties(0).multi_processor_count != 148 or \
+        _native.load_abi().sage_direct_takes_bf16_v(B, Hq, Sq, Skv, D, int(causal))
     q, k, v = (H.randn((B, h, s, D), i, torch.bfloat16).cuda() for i, (h, s) in enumerate(((Hq, Sq), (Hkv, Skv), (Hkv, Skv))))
     v[:, :, :, 5] *= 1e-7                          # fp16 subnormals
     v[0, 0, -1, 3] = 1e6                           # overflows to infinity
     if layout == "NHD":
         q, k, v = (t.transpose(1, 2).contiguous() for t in (q, k, v))
     lay = 1 if layout == "HND" else 0
-    o = sageattn(q, k, v, tensor_layout=layout, is_causal=causal)
-    o2 = torch.empty_like(q)
+    o, lse = sageattn(q, k, v, tensor_layout=layout, is_causal=causal, return_lse=True)
+    o2, lse2 = torch.empty_like(q), torch.empty_like(lse)
     try:
         H.set_streamk(0)                           # the launch ahead and the plain launch behind it
-        ops.bf16_attn(q, k, ops.v_to_f16(v, lay), o2, lay, 1, int(causal), D ** -0.5)
+        ops.bf16_attn(q, k, ops.v_to_f16(v, lay), o2, lay, 1, int(causal), D ** -0.5, lse=lse2)
     finally:
         H.set_streamk(-1)
     assert torch.equal(o.nan_to_num(7.0), o2.nan_to_num(7.0))
     assert torch.equal(o.isnan(), o2.isnan())
+    assert torch.equal(lse, lse2)
 
 
 @pytest.mark.gpu
