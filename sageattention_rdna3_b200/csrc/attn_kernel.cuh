@@ -184,14 +184,16 @@ struct Segment {
 // within a group the heaviest (last) query tiles go first and neighbouring CTAs are neighbouring
 // heads.  The CTAs resident at any moment then read the K/V of a few heads only (they stay in L2),
 // and the query heads of one KV head (GQA) run together.  The last group of a causal launch is larger.
-// (Divisions of unsigned numbers, one for both the tile and the head: the map stands ahead of the first load of
-// every item.  With signed ones 512 items of 4 tiles, un-quantised, D=128, take 24.08 instead of 23.47 us, 320 items of
-// one tile, D=64, 10.89 instead of 10.77.)
+// (The map stands ahead of the first load of every item.  With divisions of unsigned numbers, one for both the tile and the
+// head, 512 items of 4 tiles, un-quantised, D=128, take 23.47 instead of 24.08 us, 320 items of one tile, D=64, 10.77
+// instead of 10.89.  SIGNED_MAP, for the int8 kernel without a causal mask at D=64: that kernel is compiled differently around
+// the shorter map, and 1 % slower on long sequences, 16 heads of 22911 tokens 2752 us instead of 2708, 10 of 7000 182.6 instead
+// of 179.9.)
 // STREAMK = true: the KV-tile steps of all items, in (batch, head, query tile) order, form one line
 // of sk_total_tiles steps; CTA c owns steps [c*T/G, (c+1)*T/G) and walks through the items they
 // belong to: the tail of one item, whole items, the head of another.  All CTAs get the same amount
 // of work whatever the number of items is.
-template <bool CAUSAL, bool STREAMK>
+template <bool CAUSAL, bool STREAMK, bool SIGNED_MAP>
 struct SegIter {
   const AttnParams& p;
   long long t, t_end;
@@ -220,19 +222,29 @@ struct SegIter {
     if constexpr (!STREAMK) {
       if (!first) return false;
       first = false;
-      int g_first = p.tail_first, g_size = p.tail_size, within = blockIdx.x;
-      if (!CAUSAL || within < p.tail_block) {
+      if constexpr (SIGNED_MAP) {
         const int per_group = p.n_q_tiles * p.head_group;
-        const int group = static_cast<unsigned>(within) / static_cast<unsigned>(per_group);
-        g_first = group * p.head_group;
-        g_size = CAUSAL ? p.head_group : min(p.head_group, p.B * p.Hq - g_first);
-        within -= group * per_group;
+        const int group = blockIdx.x / per_group;
+        const int g_first = group * p.head_group;
+        const int g_size = min(p.head_group, p.B * p.Hq - g_first);
+        const int within = blockIdx.x - group * per_group;
+        const int qt = p.light_first ? within / g_size : p.n_q_tiles - 1 - within / g_size;
+        fill(s, g_first + within % g_size, qt);
       } else {
-        within -= p.tail_block;
+        int g_first = p.tail_first, g_size = p.tail_size, within = blockIdx.x;
+        if (!CAUSAL || within < p.tail_block) {
+          const int per_group = p.n_q_tiles * p.head_group;
+          const int group = static_cast<unsigned>(within) / static_cast<unsigned>(per_group);
+          g_first = group * p.head_group;
+          g_size = CAUSAL ? p.head_group : min(p.head_group, p.B * p.Hq - g_first);
+          within -= group * per_group;
+        } else {
+          within -= p.tail_block;
+        }
+        const int up = static_cast<unsigned>(within) / static_cast<unsigned>(g_size);
+        const int qt = p.light_first ? up : p.n_q_tiles - 1 - up;
+        fill(s, g_first + within - up * g_size, qt);
       }
-      const int up = static_cast<unsigned>(within) / static_cast<unsigned>(g_size);
-      const int qt = p.light_first ? up : p.n_q_tiles - 1 - up;
-      fill(s, g_first + within - up * g_size, qt);
       const int kv_limit = CAUSAL ? min(s.q_base + kBlockM, p.Skv) : p.Skv;   // csrc/attn_gfx11.cu:502
       s.kv_lo = 0;
       s.n_kv = (kv_limit + kBlockN - 1) / kBlockN;
@@ -291,6 +303,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
                  const AttnParams p) {
   using L = AttnSmem<D, QKF ? 2 : 1, KST>;
+  using Iter = SegIter<CAUSAL, STREAMK, !CAUSAL && !QKF && D == 64>;
   constexpr int kStages = L::kStages;
   static_assert(!(QKF && DUMP), "the int32 score dump belongs to the quantised variant");
   static_assert(!VBF || (QKF && !STREAMK), "bf16 V belongs to the plain un-quantised launch");
@@ -395,7 +408,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   }
   if (warp == 4 && elect_one()) {        // the same thread as above: elect.sync is deterministic
     // The first loads (Q and K tile 0) wait for nothing in this CTA: their latency overlaps the barrier below.
-    SegIter<CAUSAL, STREAMK> first_iter(p);
+    Iter first_iter(p);
     Segment g0;
     if (first_iter.next(g0) && g0.n_kv > 0) {
       mbar_arrive_expect_tx(q_full, L::kQBytes);
@@ -434,7 +447,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // Per segment: Q, K(first tile), then for every tile K(j+1) before V(j): K is needed first.  Q and
     // K of the CTA's first segment are already on their way.
     if (elect_one()) {
-      SegIter<CAUSAL, STREAMK> iter(p);
+      Iter iter(p);
       Segment g;
       int kt = 0, it = 0;                 // KV tiles / segments so far (constant 0 unless STREAMK)
       bool ok = true;
@@ -531,7 +544,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         tc_commit(s_full + h);
       };
 
-      SegIter<CAUSAL, STREAMK> iter(p);
+      Iter iter(p);
       Segment g;
       int kt = 0, it = 0;                 // KV tiles / segments so far (constant 0 unless STREAMK)
 #pragma unroll 1
@@ -613,7 +626,7 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const uint32_t t_o = tmem_base + lane_base + kColO;
     bool ok = true;
     int kt = 0, it = 0;                   // KV tiles / segments so far (constant 0 unless STREAMK)
-    SegIter<CAUSAL, STREAMK> iter(p);
+    Iter iter(p);
     Segment sg;
 #pragma unroll 1
     while (ok && iter.next(sg)) {
