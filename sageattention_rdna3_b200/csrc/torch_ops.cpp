@@ -300,6 +300,17 @@ at::Tensor qk_int8_sv_f16_attn(const at::Tensor& q_i8, const at::Tensor& k_i8, c
   return int8_attn(q_i8, k_i8, v, o, q_scale, k_scale, layout, is_causal, value_layout, s_dump, status, lse, peer_ptrs);
 }
 
+// Whether the address ranges of two tensors have a byte in common.
+bool spans_meet(const at::Tensor& a, const at::Tensor& b) {
+  auto end = [](const at::Tensor& t) {
+    int64_t last = 0;
+    for (int64_t i = 0; i < t.dim(); ++i) last += (t.size(i) - 1) * t.stride(i);
+    return static_cast<const char*>(t.data_ptr()) + (last + 1) * t.element_size();
+  };
+  if (a.numel() == 0 || b.numel() == 0) return false;
+  return static_cast<const char*>(a.data_ptr()) < end(b) && static_cast<const char*>(b.data_ptr()) < end(a);
+}
+
 // fp16_attn / bf16_attn(Tensor query, Tensor key, Tensor value, Tensor(a!) output, int tensor_layout,
 //                       int value_layout, int is_causal, float sm_scale, int bm_sel, Tensor? status,
 //                       Tensor? lse) -> Tensor
@@ -307,19 +318,21 @@ at::Tensor qk_int8_sv_f16_attn(const at::Tensor& q_i8, const at::Tensor& k_i8, c
 // for short sequences.  query/key are fp16 (fp16_attn) or bf16 (bf16_attn) in `tensor_layout`;
 // `value` is fp16 [..,S,D] in `value_layout` (the reference passes the transposed fp16 V_T);
 // `bm_sel` picked a tile height on RDNA3 and is accepted and ignored.
-at::Tensor direct_attn(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, at::Tensor& o, int64_t layout,
+// `convert_v` (not of the operators): a bf16 value is converted ahead of the launch or inside it; `foreign_out`: output
+// is the caller's.
+at::Tensor direct_attn(const at::Tensor& q, const at::Tensor& k, const at::Tensor& value, at::Tensor& o, int64_t layout,
                        int64_t value_layout, int64_t is_causal, double sm_scale, int64_t /*bm_sel*/,
                        const c10::optional<at::Tensor>& status, const c10::optional<at::Tensor>& lse,
                        at::ScalarType want, const char* name, at::OptionalIntArrayRef peer_ptrs = c10::nullopt,
-                       bool bf16_v = false) {
+                       bool convert_v = false, bool foreign_out = false) {
   TORCH_CHECK(q.scalar_type() == want && k.scalar_type() == want && o.scalar_type() == want, name,
               ": query, key and output must be ", want);
-  TORCH_CHECK(v.scalar_type() == (bf16_v ? at::kBFloat16 : at::kHalf), name, ": value must be fp16 (convert bf16 with v_to_f16)");
+  TORCH_CHECK(convert_v || value.scalar_type() == at::kHalf, name, ": value must be fp16 (convert bf16 with v_to_f16)");
   check_16b(q, "query");
   check_16b(k, "key");
-  check_16b(v, "value");
+  check_16b(value, "value");
   check_16b(o, "output");
-  const Dims dq = dims_of(q, layout), dk = dims_of(k, layout), dv = dims_of(v, value_layout), d_o = dims_of(o, layout);
+  const Dims dq = dims_of(q, layout), dk = dims_of(k, layout), dv = dims_of(value, value_layout), d_o = dims_of(o, layout);
   TORCH_CHECK(dk.B == dq.B && dk.D == dq.D, "query/key batch or head_dim mismatch");
   TORCH_CHECK(dv.B == dk.B && dv.H == dk.H && dv.S == dk.S && dv.D == dk.D, "value shape does not match key");
   TORCH_CHECK(d_o.B == dq.B && d_o.H == dq.H && d_o.S == dq.S && d_o.D == dq.D, "output shape does not match query");
@@ -337,9 +350,18 @@ at::Tensor direct_attn(const at::Tensor& q, const at::Tensor& k, const at::Tenso
     lse_ptr = lse->data_ptr<float>();
   }
   c10::cuda::CUDAGuard guard(q.device());
+  const bool scatter = peer_ptrs.has_value() && !peer_ptrs->empty();
+  at::Tensor v = value;
+  // (a V that the output overwrites is copied ahead of the launch: its CTAs do not wait for one another)
+  const bool v_inside = convert_v && value.scalar_type() == at::kBFloat16 && !scatter && !(foreign_out && spans_meet(o, value)) &&
+                        sage_direct_takes_bf16_v((int)dq.B, (int)dq.H, (int)dq.S, (int)dk.S, (int)dq.D, (int)is_causal);
+  if (convert_v && !v_inside) {
+    v = v_to_f16(value, value_layout);
+    value_layout = kHND;
+  }
   const sage_strided_t qs = strided_of(q, layout), ks = strided_of(k, layout), vs = strided_of(v, value_layout);
   const sage_strided_t os = strided_of(o, layout);
-  if (peer_ptrs.has_value() && !peer_ptrs->empty()) {
+  if (scatter) {
     std::vector<void*> peers;
     for (int64_t a : *peer_ptrs) peers.push_back(reinterpret_cast<void*>(static_cast<uintptr_t>(a)));
     check_rc(sage_direct_attn_scatter(&qs, &ks, &vs, o.data_ptr(), os.stride_b, os.stride_h, os.stride_s, dtype_code(q),
@@ -349,7 +371,7 @@ at::Tensor direct_attn(const at::Tensor& q, const at::Tensor& k, const at::Tenso
              name);
     return o;
   }
-  if (bf16_v) {
+  if (v_inside) {
     check_rc(sage_direct_attn_bf16_v(&qs, &ks, &vs, o.data_ptr(), os.stride_b, os.stride_h, os.stride_s, (int)dq.B, (int)dq.H,
                                      (int)dk.H, (int)dq.S, (int)dk.S, (int)dq.D, (int)is_causal, (float)sm_scale, lse_ptr,
                                      status_ptr, current_stream(q)),
@@ -378,17 +400,6 @@ at::Tensor bf16_attn(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
                      "bf16_attn");
 }
 
-// Whether the address ranges of two tensors have a byte in common.
-bool spans_meet(const at::Tensor& a, const at::Tensor& b) {
-  auto end = [](const at::Tensor& t) {
-    int64_t last = 0;
-    for (int64_t i = 0; i < t.dim(); ++i) last += (t.size(i) - 1) * t.stride(i);
-    return static_cast<const char*>(t.data_ptr()) + (last + 1) * t.element_size();
-  };
-  if (a.numel() == 0 || b.numel() == 0) return false;
-  return static_cast<const char*>(a.data_ptr()) < end(b) && static_cast<const char*>(b.data_ptr()) < end(a);
-}
-
 // sageattn_fwd(Tensor query, Tensor key, Tensor value, int tensor_layout, int is_causal, float sm_scale,
 //              int smooth_k, int use_direct, Tensor status, Tensor? lse, Tensor? out, int[]? peer_ptrs) -> Tensor[]
 // The whole of the reference's sageattn body after its assertions (sageattention/core.py:96-201) in
@@ -400,8 +411,6 @@ std::vector<at::Tensor> sageattn_fwd(const at::Tensor& q, const at::Tensor& k, c
                                      int64_t is_causal, double sm_scale, int64_t smooth_k, int64_t use_direct,
                                      const at::Tensor& status, const c10::optional<at::Tensor>& lse,
                                      const c10::optional<at::Tensor>& out, at::OptionalIntArrayRef peer_ptrs) {
-  // (also for the choice of the launch, which asks for the number of SMs)
-  c10::cuda::CUDAGuard guard(q.device());
   at::Tensor o;
   if (out.has_value()) {
     TORCH_CHECK(out->sizes() == q.sizes() && out->scalar_type() == q.scalar_type() && out->device() == q.device(),
@@ -414,21 +423,12 @@ std::vector<at::Tensor> sageattn_fwd(const at::Tensor& q, const at::Tensor& k, c
   const bool bf16 = q.scalar_type() == at::kBFloat16;
   const c10::optional<at::Tensor> st(status), none;
   if (use_direct) {
-    const Dims dq = dims_of(q, layout), dv = dims_of(v, layout);
-    // (a V that the output overwrites is copied ahead of the launch: its CTAs do not wait for one another)
-    if (bf16 && v.scalar_type() == at::kBFloat16 && (!peer_ptrs.has_value() || peer_ptrs->empty()) &&
-        !(out.has_value() && spans_meet(o, v)) &&
-        sage_direct_takes_bf16_v((int)dq.B, (int)dq.H, (int)dq.S, (int)dv.S, (int)dq.D, (int)is_causal)) {
-      direct_attn(q, k, v, o, layout, layout, is_causal, sm_scale, 0, st, lse, at::kBFloat16, "bf16_attn", c10::nullopt, true);
-    } else if (bf16) {
-      direct_attn(q, k, v_to_f16(v, layout), o, layout, kHND, is_causal, sm_scale, 0, st, lse, at::kBFloat16, "bf16_attn",
-                  peer_ptrs);
-    } else {
-      direct_attn(q, k, v, o, layout, layout, is_causal, sm_scale, 0, st, lse, at::kHalf, "fp16_attn", peer_ptrs);
-    }
+    direct_attn(q, k, v, o, layout, layout, is_causal, sm_scale, 0, st, lse, bf16 ? at::kBFloat16 : at::kHalf,
+                bf16 ? "bf16_attn" : "fp16_attn", peer_ptrs, bf16, out.has_value());
     return {o};
   }
   const Dims dk_all = dims_of(k, layout);
+  c10::cuda::CUDAGuard guard(q.device());
   if (smooth_k && sage_prep_smooth_preferred((int)dk_all.B, (int)dk_all.H)) {
     // few heads: one launch for the mean and the quantisation against it
     std::vector<at::Tensor> parts =
