@@ -68,8 +68,8 @@ int sage_test_drop_v_load(int on);
 
 /* Launch schedule of the attention entry points: -1 = the library decides between one CTA per query
  * tile, persistent CTAs and persistent CTAs with two query tiles (default), 0 = one CTA per tile, 1 =
- * persistent CTAs of one tile wherever there is a workspace.  Process-wide; the environment variable SAGE_STREAMK=0|1, read once at
- * the first launch, sets the initial value.  Takes the place of the reference's per-launch
+ * persistent CTAs of one tile wherever there is a workspace.  Process-wide; the environment variable
+ * SAGE_STREAMK=0|1, read once at the first launch, sets the initial value.  Takes the place of the reference's per-launch
  * environment overrides of its tile choice (csrc/attn_gfx11.cu:2101-2114). */
 int sage_set_streamk(int mode);
 
@@ -128,19 +128,20 @@ int sage_qk_int8_sv_f16_attn_lse(const int8_t* q_i8, const int8_t* k_i8, const s
                                  int D, int is_causal, float* lse, int32_t* s_dump, int* status, void* stream);
 
 /* Persistent scheduling for problems that do not fill the GPU evenly.
- * No counterpart in the reference.  sage_qk_int8_sv_f16_attn gives every thread block one whole
- * 128-row query tile; a B200 runs 296 of them at a time, so 320 tiles (B=1, H=10, S=4096) take two
- * rounds.  Given a workspace, the _ws entry points cut the work into equal spans of KV-tile
- * steps instead, keep partial results (fp32) in the workspace and merge them with a second small
- * kernel; they fall back to the plain launch when that would not pay, when the workspace is NULL
- * or too small, or when s_dump is set.  (Many short items run on persistent CTAs that take whole items, two query
- * tiles at a time, with or without a workspace: the same bits as the plain launch.)  Results agree with the plain launch to fp32 rounding of
- * the merge (same int8 products, same softmax).
+ * No counterpart in the reference.  The plain launch gives every thread block one whole 128-row query tile; a B200
+ * runs 296 of them at a time, so 320 tiles (B=1, H=10, S=4096) would take two rounds.  Given a workspace, the _ws entry
+ * points cut the work, or what is left of it after whole rounds, into equal spans of KV-tile steps, on blocks of one
+ * query tile or of two, keep partial results (fp32) in the workspace and merge them with a second small kernel; they
+ * fall back to the plain launch when that would not pay, when the workspace is NULL or too small, or when s_dump is set.
+ * (Many short items run on persistent blocks that take whole items, two query tiles at a time, with or without a
+ * workspace: the same bits as the plain launch.)  Results of cut items agree with the plain launch to fp32 rounding of
+ * the merge and the rounding of P to fp16 (same int8 products, same softmax); what is not a number is the same.
  * The INT8 launch lets the query heads of a GQA group share query tiles where that gives fewer of them
  * (few queries per head, no causal mask, no s_dump, output rows that run on from one head to the next:
  * o_stride_h == Sq * o_stride_s), and cuts up the tiles that result.
  * sage_attn_workspace_bytes: the most that a _ws call with these sizes takes on the current device, whatever
- * its number of kv heads and its output strides; 0 if all of them would use the plain launch anyway.  The
+ * its number of kv heads and its output strides; 0 if none of them cuts items (the plain launch, or whole items on
+ * persistent blocks).  The
  * workspace needs no initialisation and may be reused by the next call on the same stream. */
 int64_t sage_attn_workspace_bytes(int B, int Hq, int Sq, int Skv, int D, int is_causal);
 int sage_qk_int8_sv_f16_attn_ws(const int8_t* q_i8, const int8_t* k_i8, const sage_strided_t* v16, void* o,

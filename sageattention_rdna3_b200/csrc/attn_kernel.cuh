@@ -17,7 +17,8 @@
 // Two CTAs fit on one SM (112 KB of shared memory and 256 TMEM columns each), so the tensor pipe of
 // one overlaps the softmax of the other.
 // Launch shapes: one CTA per query tile (plain), or 2 * SMs persistent CTAs that each work through an
-// equal span of KV-tile steps and leave partial results for sage_attn_merge_kernel (STREAMK).
+// equal span of KV-tile steps and leave partial results for sage_attn_merge_kernel (STREAMK).  Two query tiles per CTA are a
+// kernel of their own (sage_pair_kernel, pair_kernel.cuh).
 //
 // TMEM columns: [0,128) S as int32 / fp32, reused in place as P (fp16 pairs in columns [0,64));
 //               [128,128+D) O as fp32.
@@ -393,8 +394,9 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   // preparation): with the allocation before the wait 18 of 110 SMs got two CTAs and 38 none, after it
   // every CTA has an SM to itself, as on an idle GPU.  4 heads of 4096 tokens, D=128: 62.1 -> 48.9 us per
   // call; 6 heads of 3072, un-quantised, D=64: 44.4 -> 33.0.  Causal launches of some 400-1000 items had
-  // gained from the uneven placement, which is given up: 16 heads of 4096 tokens 82.8 -> 90.1 us (95 with
-  // ordinary launches); a persistent launch, whose CTAs all start at once, pays about 0.5 us for the allocation.
+  // gained from the uneven placement: 16 heads of 4096 tokens 82.8 -> 90.1 us (95 with ordinary launches); the larger last
+  // group of heads (sage_tail_group_first) has given that back (the attention launch 77 -> 71 us).  A persistent launch,
+  // whose CTAs all start at once, pays about 0.5 us for the allocation.
   if (warp == 5) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
@@ -996,8 +998,8 @@ sage_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 }
 
 // ---------------------------------------------------------------------------------------------
-// Merge of the partial results of the persistent variant.  One CTA per item (query tile of one
-// (batch, head)); items that one attention CTA covered completely were written by it and are
+// Merge of the partial results of the launches that cut items.  Several CTAs per item (query tile of one (batch, head),
+// or pair of them); items that one attention CTA covered completely were written by it and are
 // skipped.  For the others, part k (k = 0 .. n-1) holds o_k = acc_k / l_k and e_k = m_k + log2 l_k
 // over its share of the keys, and
 //     o = sum_k 2^(e_k - E) o_k / sum_k 2^(e_k - E),   E = max_k e_k,   lse = (E + log2 sum) ln 2.

@@ -236,9 +236,9 @@ int sm_count(int* out) {
   return SAGE_OK;
 }
 
-// Choice between the plain and the persistent launch: -1 = by the cost model, 0 = never persistent,
-// 1 = always.  SAGE_STREAMK in the environment (read once, at the first use) gives the initial
-// value; sage_set_streamk changes it afterwards.
+// Choice of the launch: -1 = by the rules (plan_pairs, then plan_streamk), 0 = one CTA per query tile, 1 = persistent CTAs
+// of one tile wherever there is a workspace.  SAGE_STREAMK in the environment (read once, at the first use) gives the
+// initial value; sage_set_streamk changes it afterwards.
 std::atomic<int> g_streamk_mode{-2};      // -2: environment not looked at yet
 int streamk_override() {
   static std::once_flag once;
@@ -254,7 +254,8 @@ int streamk_override() {
 
 // Persistent ("stream-K") scheduling.  The plain launch gives every CTA one whole item (a 128-row
 // query tile with all of its KV tiles); with two CTAs per SM that fills the GPU in waves of
-// 2 * SMs items, and a problem of 320 items (B=1, H=10, S=4096) takes two waves where 1.08 would do.
+// 2 * SMs items, and a problem of 320 items takes two waves where 1.08 would do (4 heads of 10240 tokens, D=128, un-quantised
+// or not; 10 of 4096 at D=64 have gone to plan_pairs since).
 // The persistent launch cuts the T = sum of KV-tile steps into 2 * SMs equal spans instead; a span
 // that covers part of an item leaves a partial result in the workspace and a merge kernel combines
 // them.  It costs about three KV-tile steps per CTA (a second pipeline fill and drain, the merge), so
